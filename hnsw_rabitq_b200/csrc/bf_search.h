@@ -16,9 +16,17 @@ struct BfParams {
     uint64_t* out_labels;
     float* out_dists;
     int32_t* out_counts;
-    uint32_t* status;        // bit 0x1 set when a bounded wait gives up
+    // workspace of one batch of queries (set by launch_bf_search)
+    uint32_t* keys;          // nq x count distance keys
+    uint32_t* gmin;          // nq x groups: smallest allowed key of 32 rows
+    uint32_t groups;         // ceil(count / 32)
 };
 
-cudaError_t launch_bf_search(const BfParams& p, int space, int num_sms, cudaStream_t stream);
+// Whether k results over rows of row_floats floats are within the interface's limits.
+bool bf_supported(uint32_t k, uint32_t row_floats, size_t max_smem);
+// Queries of p that run at once, and the bytes of workspace for `batch` at once.
+uint32_t bf_batch(const BfParams& p);
+size_t bf_workspace(const BfParams& p, uint32_t batch);
+cudaError_t launch_bf_search(BfParams p, int space, void* workspace, uint32_t batch, cudaStream_t stream);
 
 }  // namespace hnswgpu

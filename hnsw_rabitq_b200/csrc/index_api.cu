@@ -694,6 +694,30 @@ void run_epsilon(hnswgpu_index* h, const float* dq, uint64_t nq, float eps, uint
                "hnsw_search launch");
 }
 
+// Stream-ordered workspace of one call from the index's own pool: freed on
+// the stream that used it, so calls on several streams never share a block.
+// The pool keeps its peak for the next call until the index is freed.
+struct PoolBuf {
+    void* p = nullptr;
+    cudaStream_t st;
+    explicit PoolBuf(cudaStream_t s) : st(s) {}
+    cudaError_t alloc(hnswgpu_index* h, size_t bytes) {
+        if (!h->pool) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = h->device;
+            cuda_check(cudaMemPoolCreate(&h->pool, &props), "cudaMemPoolCreate");
+            uint64_t keep = ~0ull;
+            cuda_check(cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
+        }
+        return cudaMallocFromPoolAsync(&p, bytes, h->pool, st);
+    }
+    ~PoolBuf() {
+        if (p) cudaFreeAsync(p, st);
+    }
+};
+
 // Exact brute force of a batch on device buffers (bf_search.cu).
 static void run_bf_exact(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, const uint8_t* dallow,
                          uint64_t* dl, float* dd, int32_t* dc, cudaStream_t st) {
@@ -711,8 +735,20 @@ static void run_bf_exact(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_
     b.out_labels = dl;
     b.out_dists = dd;
     b.out_counts = dc;
-    b.status = h->status.p;
-    cuda_check(hnswgpu::launch_bf_search(b, kspace(h), h->num_sms, st), "bf_search launch");
+    int max_optin = 0;
+    cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attr");
+    if (!hnswgpu::bf_supported(b.k, b.row_floats, (size_t)max_optin))
+        cuda_check(cudaErrorInvalidConfiguration, "bf_search launch");
+    uint32_t batch = hnswgpu::bf_batch(b);
+    PoolBuf ws(st);
+    cudaError_t e = ws.alloc(h, hnswgpu::bf_workspace(b, batch));
+    while (e == cudaErrorMemoryAllocation && batch > 8) {  // little memory left: fewer queries at once
+        (void)cudaGetLastError();
+        batch = std::max(8u, batch / 4);
+        e = ws.alloc(h, hnswgpu::bf_workspace(b, batch));
+    }
+    cuda_check(e, "bf_search workspace");
+    cuda_check(hnswgpu::launch_bf_search(b, kspace(h), ws.p, batch, st), "bf_search launch");
 }
 
 static uint32_t pow2_at_least(uint64_t v) {
@@ -881,23 +917,7 @@ void run_search(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint
     if (h->is_bf && prec) {
         run_bf_tc(h, dq, nq, k, rerank, dallow, dl, dd, dc, dtrace, st, prec);
     } else if (h->is_bf || scan) {
-        hnswgpu::BfParams b{};
-        b.vecs = h->vecs.p;
-        b.labels = h->dlabels.p;
-        b.allow = dallow;
-        b.count = (uint32_t)h->count;
-        b.dim = (uint32_t)h->dim;
-        b.row_floats = h->row_floats;
-        b.queries = dq;
-        b.nq = (uint32_t)nq;
-        b.k = (uint32_t)k;
-        b.normalize = h->space == HNSWGPU_SPACE_COSINE ? 1u : 0u;
-        b.out_labels = dl;
-        b.out_dists = dd;
-        b.out_counts = dc;
-        b.status = h->status.p;
-        cuda_check(hnswgpu::launch_bf_search(b, kspace(h), h->num_sms, st),
-                   "bf_search launch");
+        run_bf_exact(h, dq, nq, k, dallow, dl, dd, dc, st);
     } else {
         run_hnsw(h, dq, nq, k, ef, dallow, dl, dd, dc, dtrace, st, exact, prec, rerank, term, replay_all);
     }

@@ -78,6 +78,7 @@ struct hnswgpu_index {
     DevBuf<uint32_t> links0, upper_off, upper_links, deleted_bits;
     DevBuf<uint64_t> dlabels;
     DevBuf<uint32_t> docs;  // multi-vector index: document id per element (else empty)
+    cudaMemPool_t pool = nullptr;  // stream-ordered per-call workspaces (PoolBuf)
     // per-call workspace
     DevBuf<uint32_t> counters;  // ring of work counters
     uint32_t next_counter = 0;
@@ -119,6 +120,7 @@ struct hnswgpu_index {
     ~hnswgpu_index() {
         if (tie_host) cudaFreeHost(tie_host);
         if (tie_ev) cudaEventDestroy(tie_ev);
+        if (pool) cudaMemPoolDestroy(pool);
     }
     uint64_t device_bytes() const {
         return vecs.bytes() + links0.bytes() + upper_off.bytes() + upper_links.bytes() + deleted_bits.bytes() +
