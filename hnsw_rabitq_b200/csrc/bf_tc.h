@@ -14,14 +14,16 @@ struct TcArgs {
     uint32_t n_rows;           // rows of the row map (the sample in MODE 1)
     uint64_t row_step;         // global row id = map row x row_step
     uint32_t k_blocks;         // 128-byte K blocks per row
-    uint32_t chunk_tiles;      // MODE 0: 256-row tiles per work item
+    uint32_t chunk_tiles;      // 256-row tiles per work item
     const float2* rowinfo;     // per map row: (|x|^2, scale), padded to whole 256-row tiles
     const float* qscale;       // per query: scale of its low-precision row
     const uint8_t* allow;      // optional per-row mask
-    float* tau;                // per query: threshold (MODE 0 reads, MODE 1 writes)
+    const float* tau;          // MODE 0: threshold per query
+    float* part;               // MODE 1: ascending 16 best per query, chunk and tile half
     uint32_t* cnt;             // MODE 0: candidates per query
     uint64_t* buf;             // MODE 0: nq x cap (distance key << 32 | row)
     uint32_t cap;
+    uint32_t stop_full;        // MODE 0: stop collecting for a query whose list overflowed
     uint32_t* status;
 };
 
@@ -40,6 +42,11 @@ struct TcSelectArgs {
 };
 
 size_t tc_smem_bytes();
+// Threshold pass over n_sample rows: lists per query and tiles per work item;
+// floats of its scratch; the thresholds from the lists.
+uint32_t tc_tau_lists(uint32_t n_sample, uint32_t* chunk_tiles);
+size_t tc_tau_part(uint32_t nq, uint32_t lists);
+cudaError_t launch_tc_tau(const float* part, uint32_t nq, uint32_t lists, float* tau, cudaStream_t st);
 cudaError_t launch_fp64_distances(const float* q, uint64_t nq, uint32_t m, uint32_t dim, const float* vecs,
                                   uint32_t row_floats, const uint32_t* rows, int space, int normalize, double* out,
                                   cudaStream_t st);

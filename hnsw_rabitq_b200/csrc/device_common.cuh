@@ -292,6 +292,21 @@ __device__ __forceinline__ float group4_dist16(const float* __restrict__ q, cons
     return group4_reduce<SPACE>(c0, c1, c2, c3);
 }
 
+// GCC's _mm512_reduce_add_ps tree over the 16 accumulators of a 4-lane group.
+__device__ __forceinline__ float group4_ip_sum(float c0, float c1, float c2, float c3) {
+    // T3[i] = a[i+8] + a[i]: lanes 0,1 pair with lanes 2,3
+    float u0 = __fadd_rn(__shfl_down_sync(FULL, c0, 2), c0);
+    float u1 = __fadd_rn(__shfl_down_sync(FULL, c1, 2), c1);
+    float u2 = __fadd_rn(__shfl_down_sync(FULL, c2, 2), c2);
+    float u3 = __fadd_rn(__shfl_down_sync(FULL, c3, 2), c3);
+    // T6[i] = T3[i+4] + T3[i]: lane 0 pairs with lane 1
+    float v0 = __fadd_rn(__shfl_down_sync(FULL, u0, 1), u0);
+    float v1 = __fadd_rn(__shfl_down_sync(FULL, u1, 1), u1);
+    float v2 = __fadd_rn(__shfl_down_sync(FULL, u2, 1), u2);
+    float v3 = __fadd_rn(__shfl_down_sync(FULL, u3, 1), u3);
+    return __fadd_rn(__fadd_rn(v0, v2), __fadd_rn(v1, v3));
+}
+
 // Cross-lane reduction of group4_dist16: lane a of a 4-lane group holds the
 // reference's accumulators 4a .. 4a+3.
 template <int SPACE>
@@ -310,17 +325,7 @@ __device__ __forceinline__ float group4_reduce(float c0, float c1, float c2, flo
         r = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(r, f0), f1), f2), f3);
         return r;
     } else {
-        // T3[i] = a[i+8] + a[i]: lanes 0,1 pair with lanes 2,3
-        float u0 = __fadd_rn(__shfl_down_sync(FULL, c0, 2), c0);
-        float u1 = __fadd_rn(__shfl_down_sync(FULL, c1, 2), c1);
-        float u2 = __fadd_rn(__shfl_down_sync(FULL, c2, 2), c2);
-        float u3 = __fadd_rn(__shfl_down_sync(FULL, c3, 2), c3);
-        // T6[i] = T3[i+4] + T3[i]: lane 0 pairs with lane 1
-        float v0 = __fadd_rn(__shfl_down_sync(FULL, u0, 1), u0);
-        float v1 = __fadd_rn(__shfl_down_sync(FULL, u1, 1), u1);
-        float v2 = __fadd_rn(__shfl_down_sync(FULL, u2, 1), u2);
-        float v3 = __fadd_rn(__shfl_down_sync(FULL, u3, 1), u3);
-        return __fsub_rn(1.0f, __fadd_rn(__fadd_rn(v0, v2), __fadd_rn(v1, v3)));
+        return __fsub_rn(1.0f, group4_ip_sum(c0, c1, c2, c3));
     }
 }
 
@@ -328,6 +333,68 @@ template <int SPACE>
 __device__ __forceinline__ float distance(const float* q, const float* x, int dim) {
     if (SPACE == 0) return dist_l2(q, x, dim);
     return dist_ip(q, x, dim);
+}
+
+// distance() of any dimension over a group of 4 lanes (a = lane & 3), in the
+// same summation order; the reads of a group are contiguous.  All 32 lanes
+// call it with the same dim; the result is valid in lanes with a == 0.  q in
+// shared memory, x in global memory.
+template <int SPACE>
+__device__ __forceinline__ float group4_dist(const float* __restrict__ q, const float* __restrict__ x, int dim,
+                                             int a) {
+    if (dim < 4) return distance<SPACE>(q, x, dim);
+    float r;
+    int done;
+    if ((dim & 15) == 0 || (dim > 16 && (dim & 3))) {
+        // 16 accumulators over the 16-element blocks: 4 per lane
+        done = dim & ~15;
+        const float4* q4 = reinterpret_cast<const float4*>(q) + a;
+        const float4* x4 = reinterpret_cast<const float4*>(x) + a;
+        float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
+#pragma unroll 8
+        for (int c = 0; c < dim >> 4; c++) {
+            const float4 qv = q4[4 * c], xv = x4[4 * c];
+            const float t0 = SPACE == 0 ? __fsub_rn(qv.x, xv.x) : qv.x, t1 = SPACE == 0 ? __fsub_rn(qv.y, xv.y) : qv.y;
+            const float t2 = SPACE == 0 ? __fsub_rn(qv.z, xv.z) : qv.z, t3 = SPACE == 0 ? __fsub_rn(qv.w, xv.w) : qv.w;
+            c0 = __fmaf_rn(t0, SPACE == 0 ? t0 : xv.x, c0);
+            c1 = __fmaf_rn(t1, SPACE == 0 ? t1 : xv.y, c1);
+            c2 = __fmaf_rn(t2, SPACE == 0 ? t2 : xv.z, c2);
+            c3 = __fmaf_rn(t3, SPACE == 0 ? t3 : xv.w, c3);
+        }
+        r = SPACE == 0 ? group4_reduce<0>(c0, c1, c2, c3) : group4_ip_sum(c0, c1, c2, c3);
+    } else {
+        // 4 accumulators over the 4-element chunks (inner product: 8 over the
+        // 16-element blocks, folded to 4 first): lane a keeps a (and a + 4)
+        const int n4 = dim >> 2;
+        done = n4 << 2;
+        float s = 0.f;
+        if (SPACE == 0) {
+#pragma unroll 8
+            for (int c = 0; c < n4; c++) {
+                const float t = __fsub_rn(q[4 * c + a], x[4 * c + a]);
+                s = __fmaf_rn(t, t, s);
+            }
+        } else {
+            float h = 0.f;
+            const int n16 = dim >> 4;
+#pragma unroll 4
+            for (int c = 0; c < n16; c++) {
+                const float* qc = q + 16 * c + a;
+                const float* xc = x + 16 * c + a;
+                const float x0 = xc[0], x1 = xc[4], x2 = xc[8], x3 = xc[12];
+                s = __fmaf_rn(qc[0], x0, s);
+                h = __fmaf_rn(qc[4], x1, h);
+                s = __fmaf_rn(qc[8], x2, s);
+                h = __fmaf_rn(qc[12], x3, h);
+            }
+            s = __fadd_rn(s, h);
+            for (int c = 4 * n16; c < n4; c++) s = __fmaf_rn(q[4 * c + a], x[4 * c + a], s);
+        }
+        const float s1 = __shfl_down_sync(FULL, s, 1), s2 = __shfl_down_sync(FULL, s, 2), s3 = __shfl_down_sync(FULL, s, 3);
+        r = __fadd_rn(__fadd_rn(__fadd_rn(s, s1), s2), s3);
+    }
+    if (done < dim) r = __fadd_rn(r, SPACE == 0 ? l2_scalar(q + done, x + done, dim - done) : ip_scalar(q + done, x + done, dim - done));
+    return SPACE == 0 ? r : __fsub_rn(1.0f, r);
 }
 
 // normalize_vector (python_bindings/bindings.cpp:241-248), run by one lane:

@@ -818,6 +818,7 @@ void run_bf_tc(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint3
     a.cnt = h->tc_cnt.p;
     a.buf = h->tc_buf.p;
     a.cap = (uint32_t)cap;
+    a.stop_full = dtrace ? 0u : 1u;  // the trace reports how many candidates there were
     a.status = h->status.p;
     if (sampled) {
         cuda_check(hnswgpu::tc_encode_map(h->tcopy[prec].p, prec, n_sample, dim, (uint64_t)trow * step, 256, &smap),
@@ -829,8 +830,11 @@ void run_bf_tc(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint3
         t.n_rows = (uint32_t)n_sample;
         t.row_step = step;
         t.rowinfo = h->tc_sinfo.p;
-        t.chunk_tiles = 1;
+        const uint32_t lists = hnswgpu::tc_tau_lists(t.n_rows, &t.chunk_tiles);
+        h->tc_part.ensure(hnswgpu::tc_tau_part(t.nq, lists));
+        t.part = h->tc_part.p;
         cuda_check(hnswgpu::launch_tc_scores(qmap, smap, t, prec, space, 1, h->num_sms, st), "threshold launch");
+        cuda_check(hnswgpu::launch_tc_tau(t.part, t.nq, lists, h->tc_tau.p, st), "threshold merge launch");
     } else {
         cuda_check(hnswgpu::launch_tc_fill(h->tc_tau.p, nq, __builtin_inff(), st), "fill launch");
     }

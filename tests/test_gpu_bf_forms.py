@@ -72,3 +72,42 @@ def test_query_batches(tmp_path):
     x = rng.standard_normal((70000, 4)).astype(np.float32)
     g, o = _pair(tmp_path, x, "cosine")
     _same(g, o, rng.standard_normal((1001, 4)).astype(np.float32), 10)
+
+
+@pytest.mark.parametrize("prec", ["bf16", "fp8"])
+@pytest.mark.parametrize("space", ["l2", "ip"])
+@pytest.mark.parametrize("dim", [2, 5, 16, 20, 33, 100, 129])
+def test_rerank_forms(prec, space, dim):
+    """Every row re-ranked: the low-precision scan is the exact one."""
+    rng = np.random.default_rng(dim)
+    x = rng.standard_normal((1000, dim)).astype(np.float32)
+    q = rng.standard_normal((130, dim)).astype(np.float32)
+    g = H.BFIndex(space, dim)
+    g.init_index(1000)
+    g.add_items(x, rng.permutation(1000))
+    el, ed = g.knn_query(q, k=10)
+    l, d, c, _ = g.knn_query_traced(q, 10, precision=prec, rerank=1000)
+    assert np.array_equal(l, el) and np.array_equal(d.view(np.uint32), ed.view(np.uint32))
+
+
+@pytest.mark.parametrize("prec", ["bf16", "fp8"])
+def test_lists_that_overflow(prec):
+    """Queries whose candidate list overflows are answered exactly: many tied
+    rows under the threshold, and a sample without any admissible row."""
+    rng = np.random.default_rng(7)
+    x = rng.integers(0, 2, (60000, 16)).astype(np.float32)
+    x[::2] = 1.0
+    q = rng.integers(0, 2, (300, 16)).astype(np.float32)
+    g = H.BFIndex("l2", 16)
+    g.init_index(60000)
+    g.add_items(x)
+    for filt in (None, lambda v: v % 12 != 0 and v % 15 != 0):
+        g.precision = "fp32"
+        el, ed = g.knn_query(q, k=10, filter=filt)
+        g.precision = prec
+        l, d = g.knn_query(q, k=10, filter=filt)
+        lt, dt, _, tr = g.knn_query_traced(q, 10, filter=filt, precision=prec)
+        assert np.array_equal(l, lt) and np.array_equal(d, dt)
+        redo = tr[:, 2] == 1
+        assert redo.any()
+        assert np.array_equal(l[redo], el[redo]) and np.array_equal(d[redo], ed[redo])
