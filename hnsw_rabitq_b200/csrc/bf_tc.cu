@@ -83,10 +83,10 @@ __device__ unsigned long long g_tc_timing[256][10];
 #endif
 
 struct TcSmem {
-    float2 hinfo[2][kTileN];  // per-row helpers of the tiles in the two accumulators
-    // candidates of the current / previous tile, slot-major (a warp's stores
-    // hit distinct banks); the extra slot takes what no longer fits
-    uint64_t cst[2][kStageC + 1][kEpiThreads];
+    alignas(16) float2 hinfo[2][kTileN];  // per-row helpers of the tiles in the two accumulators
+    // (distance, column) candidates of the current / previous tile, slot-major
+    // (a warp's stores hit distinct banks)
+    uint64_t cst[2][kStageC][kEpiThreads];
     uint64_t full[kStages], empty[kStages], tfull[2], tempty[2], done;
     uint64_t afull, aempty;  // resident query tile loaded / no longer read by the MMAs
     uint32_t tmem, error;
@@ -152,15 +152,16 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                  : "memory");
 }
 
-// 64 consecutive fp32 accumulator columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float* v) {
-    uint32_t r[64];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+// 32 consecutive fp32 accumulator columns of this thread's TMEM lane: the load
+// is only issued; the values are there after tmem_wait32 on the same array
+// (whose operands keep every use behind the wait).
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                  : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 64; i++) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_wait32(uint32_t (&r)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])::"memory");
 }
 
 // One accumulator column of this thread's TMEM lane (whole warp).
@@ -372,22 +373,34 @@ __global__ void __launch_bounds__(kThreads, 1)
             // candidates of a tile are staged, then claimed with one atomic
             // whose result is used a tile later (its latency hidden)
             int cb_cur = 0, n_prev = 0;
-            uint32_t prev_slot = 0;
+            uint32_t prev_slot = 0, prev_row0 = 0;
+            // a staged (distance, column) as the list's (distance key, row)
+            auto staged = [&](uint64_t e, uint32_t first) {
+                return mkkey(__uint_as_float((uint32_t)e), (uint32_t)((uint64_t)(first + (uint32_t)(e >> 32)) * a.row_step));
+            };
             float top[kTopT];
 #pragma unroll
             for (int i = 0; i < kTopT; i++) top[i] = inf;
             const uint32_t t_end = min(n_tiles, (ck + 1) * chunk);
+            bool pass[4];
+            auto fetch_mask = [&](uint32_t t) {
+#pragma unroll
+                for (int w = 0; w < 4; w++) {
+                    const uint32_t lr = t * kTileN + (uint32_t)(half * 128 + w * 32 + lane);
+                    pass[w] = lr < a.n_rows && (!a.allow || a.allow[(uint64_t)lr * a.row_step]);
+                }
+            };
             for (uint32_t t = ck * chunk; t < t_end; t++) {
                 // columns of this half that are rows of the map and pass the
-                // mask (a lane holds all four words)
+                // mask (every lane holds all four words); the mask bytes of
+                // the next tile are fetched a tile ahead
+                const bool masked = a.allow || t == n_tiles - 1;
                 uint32_t cm[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-                if (a.allow || t == n_tiles - 1) {
+                if (masked) {
+                    if (!a.allow || t == ck * chunk) fetch_mask(t);
 #pragma unroll
-                    for (int w = 0; w < 4; w++) {
-                        const uint32_t lr = t * kTileN + (uint32_t)(half * 128 + w * 32 + lane);
-                        const bool in = lr < a.n_rows && (!a.allow || a.allow[(uint64_t)lr * a.row_step]);
-                        cm[w] = __ballot_sync(FULL, in);
-                    }
+                    for (int w = 0; w < 4; w++) cm[w] = __ballot_sync(FULL, pass[w]);
+                    if (a.allow && t + 1 < t_end) fetch_mask(t + 1);
                 }
                 const long long w3 = clock64();
                 if (!tc_wait(&s.tfull[acc], aphase)) {
@@ -399,98 +412,106 @@ __global__ void __launch_bounds__(kThreads, 1)
                 tc_fence_after();
                 const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * kTileN;
                 const float2* hinfo = s.hinfo[acc];
-                auto dist_of = [&](float sc, int col) {
+                auto dist_with = [&](float sc, const float2& h) {
                     if (!NEEDH) return sc * coef;
-                    const float2 h = hinfo[col];  // one broadcast shared-memory load
                     const float sv = PREC == 1 ? sc : sc * h.y;
                     return SPACE == 0 ? fmaf(sv, coef, h.x) : sv * coef;
+                };
+                auto dist_of = [&](float sc, int col) {
+                    return dist_with(sc, NEEDH ? hinfo[col] : make_float2(0.f, 0.f));
                 };
                 uint64_t* slots = &s.cst[cb_cur][0][et];
                 const uint32_t slot0 = smem_u32(slots), full = slot0 + kStageC * kSlotBytes;
                 uint32_t slot = slot0;  // MODE 0: where this thread's next candidate goes
-                // valid staged candidates [0, n) of this tile as (distance key,
-                // row) at the front; returns their number
+                const uint32_t row0 = t * kTileN + (uint32_t)half * 128;  // row of the map at column 0 of this half
+                // masked tiles: drop the staged candidates [0, n) whose column
+                // is masked; returns how many are left at the front
                 auto compact = [&](int n) {
+                    if (!masked) return n;
                     int m = 0;
                     for (int i = 0; i < n; i++) {
                         const uint64_t e = slots[(size_t)i * kEpiThreads];
-                        const uint32_t col = (uint32_t)(e >> 32) & 127u;
+                        const uint32_t col = (uint32_t)(e >> 32);
                         const uint32_t w = col < 32 ? cm[0] : col < 64 ? cm[1] : col < 96 ? cm[2] : cm[3];
-                        if (!((w >> (col & 31)) & 1u)) continue;
-                        const uint32_t row = (uint32_t)((uint64_t)(t * kTileN + half * 128 + col) * a.row_step);
-                        slots[(size_t)m++ * kEpiThreads] = mkkey(__uint_as_float((uint32_t)e), row);
+                        if ((w >> (col & 31)) & 1u) slots[(size_t)m++ * kEpiThreads] = e;
                     }
                     return m;
                 };
-#pragma unroll 1
-                for (int cb = 2 * half; cb < 2 * half + 2; cb++) {
-                    float v[64];
-#ifdef HNSWGPU_TC_TIMING
-                    const long long l0 = clock64();
-#endif
-                    tmem_ld64(taddr + (uint32_t)(cb * 64), v);
-#ifdef HNSWGPU_TC_TIMING
-                    if (lane == 0) TCT_ADD(8, clock64() - l0);
-#endif
+                uint32_t regs[2][32];
+                tmem_ld32(taddr + (uint32_t)(half * 128), regs[0]);
+#pragma unroll
+                for (int cb = 0; cb < 4; cb++) {
+                    uint32_t (&v)[32] = regs[cb & 1];
+                    tmem_wait32(v);
+                    if (cb < 3) tmem_ld32(taddr + (uint32_t)(half * 128 + (cb + 1) * 32), regs[(cb + 1) & 1]);
+                    const int col0 = half * 128 + cb * 32;
                     if (MODE == 0) {
                         // Straight-line: every column's distance, and a
                         // predicated store of (distance, column) for those
                         // under the threshold.  No branch and no second read
-                        // of the scores, so the cost does not grow with the
-                        // candidates of the warp's 32 queries.
+                        // of the scores; one add is all that carries from
+                        // column to column (with the compares of 8 columns
+                        // ahead of it: column by column the predicates'
+                        // latency made 40 cycles of each).
                         const uint32_t before = slot;
 #pragma unroll
-                        for (int j = 0; j < 64; j++) {
-                            const float dd = dist_of(v[j], cb * 64 + j);
-                            asm volatile(
-                                "{\n\t.reg .pred p;\n\tsetp.le.f32 p, %1, %2;\n\t"
-                                "@p st.shared.v2.f32 [%0], {%1, %3};\n\t"
-                                "@p add.u32 %0, %0, %4;\n\t@p min.u32 %0, %0, %5;\n\t}"
-                                : "+r"(slot)
-                                : "f"(dd), "f"(tau), "f"(__int_as_float((cb * 64 + j) & 127)), "n"(kSlotBytes), "r"(full)
-                                : "memory");
+                        for (int g = 0; g < 32; g += 8) {
+                            float dd[8];
+                            bool hit[8];
+#pragma unroll
+                            for (int j = 0; j < 8; j += 2) {
+                                float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+                                if (NEEDH) h = *reinterpret_cast<const float4*>(hinfo + col0 + g + j);
+                                dd[j] = dist_with(__uint_as_float(v[g + j]), make_float2(h.x, h.y));
+                                dd[j + 1] = dist_with(__uint_as_float(v[g + j + 1]), make_float2(h.z, h.w));
+                            }
+#pragma unroll
+                            for (int j = 0; j < 8; j++) hit[j] = dd[j] <= tau;
+#pragma unroll
+                            for (int j = 0; j < 8; j++) {
+                                if (hit[j] && slot < full)
+                                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(slot), "f"(dd[j]),
+                                                 "r"(cb * 32 + g + j));
+                                slot += hit[j] ? kSlotBytes : 0u;
+                            }
                         }
-                        if (!__any_sync(FULL, slot == full)) continue;
-                        // some query of this warp filled its slots: hand over
+                        if (!__any_sync(FULL, slot > full)) continue;
+                        // some query of this warp ran out of slots: hand over
                         // what was staged before this block, then append this
                         // block's candidates one column at a time
                         const int n = compact((int)((before - slot0) / kSlotBytes));
                         if (n) {
                             const uint32_t at = atomicAdd(a.cnt + q, (uint32_t)n);
                             for (int i = 0; i < n; i++)
-                                if (at + i < a.cap) a.buf[(size_t)q * a.cap + at + i] = slots[(size_t)i * kEpiThreads];
+                                if (at + i < a.cap) a.buf[(size_t)q * a.cap + at + i] = staged(slots[(size_t)i * kEpiThreads], row0);
                         }
                         slot = slot0;
                     }
-                    // (1) unrolled and small: a mask of the columns under the threshold
+                    // a mask of the columns under the threshold
                     const float thr = MODE == 0 ? tau : top[kTopT - 1];
-                    uint32_t m_lo = 0, m_hi = 0;
+                    uint32_t mine = 0;
 #pragma unroll
-                    for (int j = 0; j < 64; j++) {
-                        const float dd = dist_of(v[j], cb * 64 + j);
-                        const bool p = MODE == 0 ? dd <= thr : dd < thr;
-                        if (j < 32) m_lo |= (uint32_t)p << j;
-                        else m_hi |= (uint32_t)p << (j - 32);
+                    for (int j = 0; j < 32; j++) {
+                        const float dd = dist_of(__uint_as_float(v[j]), col0 + j);
+                        mine |= (uint32_t)(MODE == 0 ? dd <= thr : dd < thr) << j;
                     }
-                    m_lo &= (cb & 1) ? cm[2] : cm[0];
-                    m_hi &= (cb & 1) ? cm[3] : cm[1];
-                    // (2) rolled, warp-uniform: each column some lane passes;
-                    // its score is read again from TMEM (one column)
-                    uint64_t any = ((uint64_t)__reduce_or_sync(0xffffffffu, m_hi) << 32) |
-                                   __reduce_or_sync(0xffffffffu, m_lo);
-                    const uint64_t mine = ((uint64_t)m_hi << 32) | m_lo;
+                    mine &= cm[cb];
+                    uint32_t at = 0;
+                    if (MODE == 0 && mine) at = atomicAdd(a.cnt + q, (uint32_t)__popc(mine));
+                    // rolled, warp-uniform: each column some lane passes; its
+                    // score is read again from TMEM (one column)
+                    uint32_t any = __reduce_or_sync(FULL, mine);
                     while (any) {
-                        const int j = __ffsll((long long)any) - 1;
+                        const int j = __ffs(any) - 1;
                         any &= any - 1;
-                        const int col = cb * 64 + j;
                         __syncwarp();  // converge after the previous iteration's divergent tail
-                        const float sc = tmem_ld1(taddr + (uint32_t)col);
-                        if (!((mine >> j) & 1)) continue;
-                        float dd = dist_of(sc, col);
+                        const float sc = tmem_ld1(taddr + (uint32_t)(col0 + j));
+                        if (!((mine >> j) & 1u)) continue;
+                        float dd = dist_of(sc, col0 + j);
                         if (MODE == 0) {
-                            const uint64_t key = mkkey(dd, (uint32_t)((uint64_t)(t * kTileN + (uint32_t)col) * a.row_step));
-                            const uint32_t at = atomicAdd(a.cnt + q, 1u);
-                            if (at < a.cap) a.buf[(size_t)q * a.cap + at] = key;
+                            if (at < a.cap)
+                                a.buf[(size_t)q * a.cap + at] = mkkey(dd, (uint32_t)((uint64_t)(row0 + cb * 32 + j) * a.row_step));
+                            at++;
                         } else if (dd < top[kTopT - 1]) {
 #pragma unroll
                             for (int i = 0; i < kTopT; i++) {
@@ -517,9 +538,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                     // claimed a tile ago), then claim this tile's
                     for (int i = 0; i < n_prev; i++)
                         if (prev_slot + i < a.cap)
-                            a.buf[(size_t)q * a.cap + prev_slot + i] = s.cst[cb_cur ^ 1][i][et];
+                            a.buf[(size_t)q * a.cap + prev_slot + i] = staged(s.cst[cb_cur ^ 1][i][et], prev_row0);
                     if (a.stop_full && n_prev && prev_slot + n_prev > a.cap) tau = -inf;
                     n_prev = compact((int)((slot - slot0) / kSlotBytes));
+                    prev_row0 = row0;
                     if (n_prev) prev_slot = atomicAdd(a.cnt + q, (uint32_t)n_prev);
                     cb_cur ^= 1;
                 }
@@ -537,7 +559,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (MODE == 0)  // the item's last claimed batch
                 for (int i = 0; i < n_prev; i++)
                     if (prev_slot + i < a.cap)
-                        a.buf[(size_t)q * a.cap + prev_slot + i] = s.cst[cb_cur ^ 1][i][et];
+                        a.buf[(size_t)q * a.cap + prev_slot + i] = staged(s.cst[cb_cur ^ 1][i][et], prev_row0);
         }
         if (lane == 0) TCT_ADD(7, clock64() - e0);
     }
@@ -551,18 +573,33 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // ---------------------------------------------------------------------------
 // Per-row helpers of the low-precision copy: (|x|^2 of the float32 row,
-// per-row scale: the fp8 row's tail, 1 for bf16).
+// per-row scale: the fp8 row's tail, 1 for bf16).  stats (bf16 only): the
+// largest row norm and the largest norm of a row's rounding error, as bits.
 __global__ void tc_rowinfo_kernel(const float* __restrict__ vecs, uint32_t count, uint32_t dim, uint32_t row_floats,
                                   const unsigned char* __restrict__ tcopy, uint32_t trow_bytes, uint32_t prec,
-                                  float2* __restrict__ out) {
+                                  float2* __restrict__ out, uint32_t* __restrict__ stats) {
     const uint64_t row = (uint64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
     if (row >= count) return;
     const float* x = vecs + row * row_floats;
-    float s = 0.f;
-    for (uint32_t i = lane; i < dim; i += 32) s = fmaf(x[i], x[i], s);
+    float s = 0.f, e = 0.f;
+    for (uint32_t i = lane; i < dim; i += 32) {
+        s = fmaf(x[i], x[i], s);
+        if (stats) {
+            const float d = x[i] - __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(tcopy + row * trow_bytes)[i]);
+            e = fmaf(d, d, e);
+        }
+    }
 #pragma unroll
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    for (int o = 16; o; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+    }
+    if (stats && lane == 0) {
+        // as integers: any NaN or infinity exceeds every finite norm
+        atomicMax(&stats[0], __float_as_uint(sqrtf(s) * 1.001f) & 0x7fffffffu);
+        atomicMax(&stats[1], __float_as_uint(sqrtf(e) * 1.001f) & 0x7fffffffu);
+    }
     if (lane == 0) {
         const float sc = prec == 2 ? *reinterpret_cast<const float*>(tcopy + row * trow_bytes + trow_bytes - 16) : 1.f;
         out[row] = make_float2(s, sc);
@@ -574,7 +611,8 @@ __global__ void tc_rowinfo_kernel(const float* __restrict__ vecs, uint32_t count
 // scale out.
 __global__ void tc_query_prep_kernel(const float* __restrict__ q, uint32_t nq, uint32_t dim, uint32_t normalize,
                                      uint32_t prec, uint32_t trow_bytes, float* __restrict__ qf,
-                                     unsigned char* __restrict__ qt, float* __restrict__ qscale) {
+                                     unsigned char* __restrict__ qt, float* __restrict__ qscale,
+                                     const uint32_t* __restrict__ stats, int space, float2* __restrict__ qinfo) {
     const uint64_t row = (uint64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
     if (row >= nq) return;
@@ -586,8 +624,40 @@ __global__ void tc_query_prep_kernel(const float* __restrict__ q, uint32_t nq, u
     unsigned char* o = qt + row * trow_bytes;
     if (prec == 1) {
         __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(o);
-        for (uint32_t i = lane; i < trow_bytes / 2; i += 32) ob[i] = __float2bfloat16_rn(i < dim ? y[i] : 0.f);
+        float s = 0.f, e = 0.f;
+        for (uint32_t i = lane; i < trow_bytes / 2; i += 32) {
+            const float v = i < dim ? y[i] : 0.f;
+            const __nv_bfloat16 b = __float2bfloat16_rn(v);
+            ob[i] = b;
+            const float d = v - __bfloat162float(b);
+            s = fmaf(v, v, s);
+            e = fmaf(d, d, e);
+        }
         if (lane == 0) qscale[row] = 1.f;
+        if (!qinfo) return;
+#pragma unroll
+        for (int of = 16; of; of >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, of);
+            e += __shfl_xor_sync(0xffffffffu, e, of);
+        }
+        if (lane == 0) {
+            // How far the tensor-core distance of any row may lie from the
+            // reference's float32 distance.  |q.x - q'.x'| <= |q - q'||x| +
+            // |q'||x - x'| for the rounded q', x' (Cauchy-Schwarz); the
+            // tensor cores' float32 accumulation: 2^-21 |q'||x'| per 16
+            // products and 32 of them over (several times an accumulation
+            // that truncates at 24 bits); the reference's own summation and
+            // the norms, at most dim / 4 + 64 roundings of 2^-24: twice that.
+            // Subnormal inputs the tensor cores may drop: the 2^-126 term.
+            const double nq = sqrt((double)s) * 1.001, dq = sqrt((double)e) * 1.001;
+            const double M = __uint_as_float(stats[0]), D = __uint_as_float(stats[1]);
+            const double eps = 1.0 / (1 << 23);
+            const double E = dq * M + (nq + dq) * D + (dim / 16 + 32) * 4.0 * eps * (nq + dq) * (M + D) +
+                             (nq + M + 1.0) * dim * 1.2e-38;
+            const double g = (dim / 4 + 64) * eps;
+            const double B = space == 0 ? 2.0 * E + g * (nq + M) * (nq + M) : E + g * nq * M + 2.0 * eps * (1.0 + nq * M);
+            qinfo[row] = make_float2(space == 0 ? s : 1.f, (float)(B * 1.001));
+        }
         return;
     }
     float amax = 0.f;
@@ -803,6 +873,132 @@ __global__ void __launch_bounds__(kSelThreads) tc_select_rerank_kernel(TcSelectA
     if (t == 0) a.out_counts[q] = (int32_t)kk;
 }
 
+// Exact form of step 3.  The candidates of a query are all rows whose bf16
+// tensor-core distance is at most tau.  With B the query's bound on how far
+// that distance lies from the reference's float32 distance (qinfo.y), and U
+// the k-th smallest exact distance among some re-ranked candidates, every row
+// of the answer has a tensor-core distance of at most U + B: the candidates up
+// to there are re-ranked too, and when U + B <= tau no row outside the list can
+// belong to the answer, which is then BruteforceSearch's own, bit for bit.
+// Otherwise (or when a list overflowed) the query is flagged for the float32
+// scan.  On unit vectors of 768 dims, k = 100, U + B reaches 2-3 k rows.
+constexpr uint32_t kCertSort = 1024;  // exact (distance, label) pairs kept
+constexpr uint32_t kCertRows = 4096;  // candidates re-ranked at once
+template <int SPACE>
+__global__ void __launch_bounds__(kSelThreads) tc_certify_kernel(TcCertArgs a) {
+    extern __shared__ __align__(1024) unsigned char sel_raw[];
+    __shared__ SelCtl c;
+    const uint32_t q = blockIdx.x;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    uint64_t* keys = reinterpret_cast<uint64_t*>(sel_raw);
+    uint64_t* el = keys + a.cap;
+    uint32_t* ek = reinterpret_cast<uint32_t*>(el + kCertSort);
+    uint32_t* rows = ek + kCertSort;
+    float* qv = reinterpret_cast<float*>(rows + kCertRows);
+    const uint32_t cnt = a.cnt[q], m = min(cnt, a.cap);
+    const float2 info = a.qinfo[q];
+    const float tau = a.tau[q];
+    auto give_up = [&]() {
+        if (t == 0) a.flags[q] = 1;
+    };
+    if (cnt > a.cap || !(info.y < 3e38f)) {
+        give_up();
+        return;
+    }
+    if (t == 0) c.n = 0;
+    for (uint32_t i = t; i < m; i += kSelThreads) keys[i] = a.buf[(size_t)q * a.cap + i];
+    for (uint32_t i = t; i < a.dim; i += kSelThreads) qv[i] = a.qf[(size_t)q * a.dim + i];
+    __syncthreads();
+    // exact keys of rows[0, n): every one into slot `at` on (bound = ~0), or
+    // those at most `bound` behind the c.n already there
+    auto rerank = [&](uint32_t n, bool keep_all, uint32_t at, uint32_t bound) {
+        for (uint32_t b = (uint32_t)warp * 8; b < n; b += kSelThreads / 4) {
+            const uint32_t i = b + (lane >> 2);
+            const uint32_t row = rows[min(i, n - 1)];
+            const float d = group4_dist<SPACE>(qv, a.vecs + (size_t)row * a.row_floats, (int)a.dim, lane & 3);
+            const uint32_t key = fkey(d);
+            if ((lane & 3) == 0 && i < n && (keep_all || key <= bound)) {
+                const uint32_t p = keep_all ? i : at + atomicAdd(&c.n, 1u);
+                if (p < kCertSort) {
+                    ek[p] = key;
+                    el[p] = a.labels[row];
+                }
+            }
+        }
+    };
+    auto sort = [&](uint32_t n) {
+        uint32_t P = 1;
+        while (P < n) P <<= 1;
+        for (uint32_t i = n + t; i < P; i += kSelThreads) {
+            ek[i] = 0xffffffffu;
+            el[i] = ~0ull;
+        }
+        __syncthreads();
+        sort_key_labels(ek, el, P);
+    };
+    const uint32_t R = min(m, a.k + a.k / 2 + 32);
+    const uint64_t thr = R < m ? select_key(keys, m, R, c) : ~0ull;
+    for (uint32_t i = t; i < m; i += kSelThreads)
+        if (keys[i] <= thr) rows[atomicAdd(&c.n, 1u)] = (uint32_t)keys[i];
+    __syncthreads();
+    rerank(R, true, 0, 0);
+    __syncthreads();
+    sort(R);
+    __syncthreads();
+    if (R < a.k) {
+        // fewer candidates than k: all the rows there are, or the list is short
+        if (tau < __int_as_float(0x7f800000)) {
+            give_up();
+            return;
+        }
+    } else {
+        const uint32_t U = ek[a.k - 1];
+        const double limit = (double)funkey(U) + (double)info.y - (double)info.x;
+        if (!(limit <= (double)tau)) {
+            give_up();
+            return;
+        }
+        if (t == 0) c.n = 0;
+        __syncthreads();
+        for (uint32_t i = t; i < m; i += kSelThreads)
+            if (keys[i] > thr && (double)funkey(khi(keys[i])) <= limit) {
+                const uint32_t p = atomicAdd(&c.n, 1u);
+                if (p < kCertRows) rows[p] = (uint32_t)keys[i];
+            }
+        __syncthreads();
+        const uint32_t n2 = c.n;
+        __syncthreads();
+        if (n2 > kCertRows) {
+            give_up();
+            return;
+        }
+        if (n2) {
+            if (t == 0) c.n = 0;
+            __syncthreads();
+            rerank(n2, false, R, U);
+            __syncthreads();
+            const uint32_t n = R + c.n;
+            if (n > kCertSort) {
+                give_up();
+                return;
+            }
+            if (n > R) {
+                sort(n);
+                __syncthreads();
+            }
+        }
+    }
+    const uint32_t kk = min(a.k, R);
+    for (uint32_t x = t; x < a.k; x += kSelThreads) {
+        a.out_labels[(size_t)q * a.k + x] = x < kk ? el[x] : ~0ull;
+        a.out_dists[(size_t)q * a.k + x] = x < kk ? funkey(ek[x]) : __int_as_float(0x7f800000);
+    }
+    if (t == 0) {
+        a.out_counts[q] = (int32_t)kk;
+        a.flags[q] = 0;
+    }
+}
+
 __global__ void tc_gather_rows_kernel(const float* __restrict__ src, const uint32_t* __restrict__ idx, uint32_t n,
                                       uint32_t dim, float* __restrict__ dst) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -945,16 +1141,18 @@ cudaError_t launch_tc_tau(const float* part, uint32_t nq, uint32_t lists, float*
 
 cudaError_t launch_tc_rowinfo(const float* vecs, uint32_t count, uint32_t dim, uint32_t row_floats,
                               const unsigned char* tcopy, uint32_t trow_bytes, uint32_t prec, float2* out,
-                              cudaStream_t st) {
+                              uint32_t* stats, cudaStream_t st) {
     if (!count) return cudaSuccess;
-    tc_rowinfo_kernel<<<(count + 7) / 8, 256, 0, st>>>(vecs, count, dim, row_floats, tcopy, trow_bytes, prec, out);
+    tc_rowinfo_kernel<<<(count + 7) / 8, 256, 0, st>>>(vecs, count, dim, row_floats, tcopy, trow_bytes, prec, out, stats);
     return cudaGetLastError();
 }
 
 cudaError_t launch_tc_query_prep(const float* q, uint32_t nq, uint32_t dim, uint32_t normalize, uint32_t prec,
-                                 uint32_t trow_bytes, float* qf, unsigned char* qt, float* qscale, cudaStream_t st) {
+                                 uint32_t trow_bytes, float* qf, unsigned char* qt, float* qscale, const uint32_t* stats,
+                                 int space, float2* qinfo, cudaStream_t st) {
     if (!nq) return cudaSuccess;
-    tc_query_prep_kernel<<<(nq + 7) / 8, 256, 0, st>>>(q, nq, dim, normalize, prec, trow_bytes, qf, qt, qscale);
+    tc_query_prep_kernel<<<(nq + 7) / 8, 256, 0, st>>>(q, nq, dim, normalize, prec, trow_bytes, qf, qt, qscale, stats,
+                                                       space, qinfo);
     return cudaGetLastError();
 }
 
@@ -988,6 +1186,20 @@ cudaError_t launch_tc_select(const TcSelectArgs& a, int space, cudaStream_t st) 
     if (!a.nq) return cudaSuccess;
     const size_t smem = tc_select_smem(a.sort_cap, a.dim, a.R);
     auto fn = space == 0 ? tc_select_rerank_kernel<0> : tc_select_rerank_kernel<1>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    fn<<<a.nq, kSelThreads, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
+size_t tc_certify_smem(uint32_t cap, uint32_t dim) {
+    return (size_t)cap * 8 + kCertSort * 12 + kCertRows * 4 + ((dim + 3) & ~3u) * 4;
+}
+
+cudaError_t launch_tc_certify(const TcCertArgs& a, int space, cudaStream_t st) {
+    if (!a.nq) return cudaSuccess;
+    const size_t smem = tc_certify_smem(a.cap, a.dim);
+    auto fn = space == 0 ? tc_certify_kernel<0> : tc_certify_kernel<1>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     fn<<<a.nq, kSelThreads, smem, st>>>(a);

@@ -41,6 +41,25 @@ struct TcSelectArgs {
     uint32_t* trace;           // optional: 4 per query, [0] = candidates found
 };
 
+// Exact scan: the candidates of the bf16 scores pass, certified.
+struct TcCertArgs {
+    uint32_t nq, k, cap, dim, row_floats;  // k <= kCertMaxK
+    const uint32_t* cnt;
+    const uint64_t* buf;
+    const float* tau;
+    const float2* qinfo;       // per query: (offset, bound): |tensor-core distance + offset - float32 distance| <= bound
+    const float* qf;
+    const float* vecs;
+    const uint64_t* labels;
+    uint64_t* out_labels;
+    float* out_dists;
+    int32_t* out_counts;
+    uint8_t* flags;            // 1: not certified, answer this query with the float32 scan
+};
+constexpr uint32_t kCertMaxK = 256;
+size_t tc_certify_smem(uint32_t cap, uint32_t dim);
+cudaError_t launch_tc_certify(const TcCertArgs& a, int space, cudaStream_t st);
+
 size_t tc_smem_bytes();
 // Threshold pass over n_sample rows: lists per query and tiles per work item;
 // floats of its scratch; the thresholds from the lists.
@@ -57,9 +76,10 @@ cudaError_t launch_tc_scores(const CUtensorMap& qm, const CUtensorMap& xm, const
                              int mode, int num_sms, cudaStream_t st);
 cudaError_t launch_tc_rowinfo(const float* vecs, uint32_t count, uint32_t dim, uint32_t row_floats,
                               const unsigned char* tcopy, uint32_t trow_bytes, uint32_t prec, float2* out,
-                              cudaStream_t st);
+                              uint32_t* stats, cudaStream_t st);
 cudaError_t launch_tc_query_prep(const float* q, uint32_t nq, uint32_t dim, uint32_t normalize, uint32_t prec,
-                                 uint32_t trow_bytes, float* qf, unsigned char* qt, float* qscale, cudaStream_t st);
+                                 uint32_t trow_bytes, float* qf, unsigned char* qt, float* qscale, const uint32_t* stats,
+                                 int space, float2* qinfo, cudaStream_t st);
 cudaError_t launch_tc_fill(float* p, uint64_t n, float v, cudaStream_t st);
 cudaError_t launch_scan_mask(const uint32_t* deleted_bits, const uint8_t* allow, uint64_t n, uint8_t* out,
                              cudaStream_t st);

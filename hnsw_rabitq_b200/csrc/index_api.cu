@@ -28,6 +28,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -718,8 +719,9 @@ struct PoolBuf {
     }
 };
 
-// Exact brute force of a batch on device buffers (bf_search.cu).
-static void run_bf_exact(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, const uint8_t* dallow,
+// Exact brute force of a batch on device buffers by the float32 kernels
+// (bf_search.cu).
+static void run_bf_simt(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, const uint8_t* dallow,
                          uint64_t* dl, float* dd, int32_t* dc, cudaStream_t st) {
     hnswgpu::BfParams b{};
     b.vecs = h->vecs.p;
@@ -757,6 +759,204 @@ static uint32_t pow2_at_least(uint64_t v) {
     return p;
 }
 
+// The low-precision copy of the rows and its per-row helpers, built once;
+// returns the copy's row pitch.
+static uint32_t ensure_tc_copy(hnswgpu_index* h, uint32_t prec) {
+    const uint64_t n = h->count;
+    const uint32_t dim = (uint32_t)h->dim;
+    ensure_traversal_copy(h, prec);
+    const uint32_t trow = hnswgpu::traversal_row_bytes(prec, dim);
+    if (h->tc_rowinfo[prec].p) return trow;
+    uint32_t* stats = nullptr;
+    if (prec == 1) {
+        h->tc_stats.ensure(2);
+        stats = h->tc_stats.p;
+        cuda_check(cudaMemsetAsync(stats, 0, 8, h->stream), "cudaMemsetAsync");
+    }
+    DevBuf<float2> info;
+    info.alloc((n + 255) / 256 * 256);  // whole tiles: read by 2 KB bulk copies
+    cuda_check(hnswgpu::launch_tc_rowinfo(h->vecs.p, (uint32_t)n, dim, h->row_floats, h->tcopy[prec].p, trow, prec, info.p,
+                                          stats, h->stream),
+               "rowinfo launch");
+    cuda_check(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    std::swap(h->tc_rowinfo[prec].p, info.p);
+    std::swap(h->tc_rowinfo[prec].n, info.n);
+    return trow;
+}
+
+static void redo_exact(hnswgpu_index* h, const float* dq, const std::vector<uint32_t>& redo, uint64_t k,
+                       const uint8_t* dallow, uint64_t* dl, float* dd, int32_t* dc, cudaStream_t st, bool tensor);
+
+// Whether the exact scan takes the tensor-core route.  Both sides measured
+// (device times): the float32 kernels run 5.3-8.1e12 elements (query x row x
+// dimension) a second; the tensor-core route costs about 80 us of launches and
+// latency and 0.1 us a query for the certification beside 0.5-1e15.  Below 8
+// queries the float32 kernels read the rows once too, without the bf16 copy.
+static bool bf_tensor_exact(uint64_t n, uint64_t nq, uint64_t k, uint64_t dim) {
+    if (k > hnswgpu::kCertMaxK || nq < 8 || nq > 0x7fffffffull || n < 4096) return false;
+    return (double)nq * (double)n * (double)dim >= 5e8 + 6e5 * (double)nq;
+}
+
+// Exact brute force through the tensor cores: bf16 scores of all rows choose
+// the candidates, exact float32 distances of these decide, and a rigorous bound
+// on the scores' error certifies that no other row can belong to the answer
+// (tc_certify_kernel).  Queries it cannot certify go to the float32 kernels.
+// 500 queries x 200k rows x 768 dims, k = 100: 9.9 ms by the float32 kernels,
+// 0.62 ms here (scores 0.17, certification 0.15, the copies).  False when there is no memory for the bf16 copy.  Synchronises.
+static bool run_bf_certified(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, const uint8_t* dallow,
+                             uint64_t* dl, float* dd, int32_t* dc, cudaStream_t st) {
+    const uint64_t n = h->count;
+    const uint32_t dim = (uint32_t)h->dim;
+    const int space = kspace(h);
+    // A sample of every step-th row: its 16th best distance has about 16 step
+    // rows at or below it, several times what the certificate reaches (2-5 k on
+    // unit vectors and Gaussian clusters).  A prime step meets every residue of
+    // the row numbers, so a periodic mask does not empty the sample.
+    // Small sets take a shorter list: at 10k rows 2000 candidates are a fifth of
+    // all rows (1000 queries x 128 dims: 0.42 ms with 2000, 0.26 ms with 500).
+    const uint64_t step = k > 100 ? 251 : (k > 25 || n >= 65536) ? 127 : 31;
+    const uint32_t cap = (uint32_t)(48 * step);
+    int max_optin = 0;
+    cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attr");
+    if (hnswgpu::tc_certify_smem(cap, dim) + 4096 > (size_t)max_optin) return false;
+    const uint64_t batch = std::min<uint64_t>(nq, 2048);
+    const uint64_t n_sample = (n + step - 1) / step;
+    uint32_t chunk_tiles = 1;
+    const uint32_t lists = hnswgpu::tc_tau_lists((uint32_t)n_sample, &chunk_tiles);
+    const uint32_t trow = hnswgpu::traversal_row_bytes(1, dim);
+    // one block of the pool holds the call's workspace
+    PoolBuf ws(st);
+    float *qf = nullptr, *qscale = nullptr, *tau = nullptr, *part = nullptr;
+    unsigned char* qt = nullptr;
+    float2 *qinfo = nullptr, *sinfo = nullptr;
+    uint32_t* cnt = nullptr;
+    uint64_t* buf = nullptr;
+    uint8_t* dflags = nullptr;
+    auto layout = [&](unsigned char* base) {
+        size_t off = 0;
+        auto take = [&](auto& p, size_t count) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + off);
+            off = (off + count * sizeof(*p) + 255) / 256 * 256;
+        };
+        take(buf, batch * cap);
+        take(qt, batch * trow + 16);
+        take(qf, batch * dim);
+        take(part, hnswgpu::tc_tau_part((uint32_t)batch, lists));
+        take(sinfo, (n_sample + 255) / 256 * 256);
+        take(qinfo, batch);
+        take(qscale, batch);
+        take(tau, batch);
+        take(cnt, batch);
+        take(dflags, nq);
+        return off;
+    };
+    try {
+        ensure_tc_copy(h, 1);
+        cuda_check(ws.alloc(h, layout(nullptr)), "exact scan workspace");
+    } catch (const ApiError& e) {
+        if (e.code != HNSWGPU_ERR_NOMEM) throw;
+        (void)cudaGetLastError();
+        return false;
+    }
+    layout(static_cast<unsigned char*>(ws.p));
+    CUtensorMap qmap, xmap, smap;
+    cuda_check(hnswgpu::tc_encode_map(h->tcopy[1].p, 1, n, dim, trow, 256, &xmap), "tensor map (rows)");
+    cuda_check(hnswgpu::tc_encode_map(h->tcopy[1].p, 1, n_sample, dim, trow * step, 256, &smap), "tensor map (sample)");
+    cuda_check(hnswgpu::launch_tc_gather_info(h->tc_rowinfo[1].p, n_sample, step, sinfo, st), "gather launch");
+    for (uint64_t b = 0; b < nq; b += batch) {
+        const uint32_t m = (uint32_t)std::min(batch, nq - b);
+        cuda_check(hnswgpu::launch_tc_query_prep(dq + b * dim, m, dim, h->space == HNSWGPU_SPACE_COSINE, 1, trow,
+                                                 qf, qt, qscale, h->tc_stats.p, space,
+                                                 qinfo, st),
+                   "query prep launch");
+        cuda_check(hnswgpu::tc_encode_map(qt, 1, m, dim, trow, 128, &qmap), "tensor map (queries)");
+        hnswgpu::TcArgs a{};
+        a.nq = m;
+        a.k_blocks = (dim * 2 + 127) / 128;
+        a.qscale = qscale;
+        a.allow = dallow;
+        a.status = h->status.p;
+        a.n_rows = (uint32_t)n_sample;
+        a.row_step = step;
+        a.rowinfo = sinfo;
+        a.chunk_tiles = chunk_tiles;
+        a.part = part;
+        cuda_check(hnswgpu::launch_tc_scores(qmap, smap, a, 1, space, 1, h->num_sms, st), "threshold launch");
+        cuda_check(hnswgpu::launch_tc_tau(a.part, m, lists, tau, st), "threshold merge launch");
+        cuda_check(cudaMemsetAsync(cnt, 0, m * 4, st), "cudaMemsetAsync");
+        a.n_rows = (uint32_t)n;
+        a.row_step = 1;
+        a.rowinfo = h->tc_rowinfo[1].p;
+        a.tau = tau;
+        a.cnt = cnt;
+        a.buf = buf;
+        a.cap = cap;
+        a.stop_full = 1;
+        // work items as in run_bf_tc, smaller where they would leave SMs idle
+        const uint64_t n_tiles = (n + 255) / 256, q_tiles = (m + 127) / 128;
+        a.chunk_tiles = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(16, n_tiles * q_tiles / (2 * (uint64_t)h->num_sms)));
+        cuda_check(hnswgpu::launch_tc_scores(qmap, xmap, a, 1, space, 0, h->num_sms, st), "scores launch");
+        hnswgpu::TcCertArgs c{};
+        c.nq = m;
+        c.k = (uint32_t)k;
+        c.cap = cap;
+        c.dim = dim;
+        c.row_floats = h->row_floats;
+        c.cnt = cnt;
+        c.buf = buf;
+        c.tau = tau;
+        c.qinfo = qinfo;
+        c.qf = qf;
+        c.vecs = h->vecs.p;
+        c.labels = h->dlabels.p;
+        c.out_labels = dl + b * k;
+        c.out_dists = dd + b * k;
+        c.out_counts = dc + b;
+        c.flags = dflags + b;
+        cuda_check(hnswgpu::launch_tc_certify(c, space, st), "certify launch");
+    }
+    // (a wait that timed out is in the status word, which the caller reads)
+    std::vector<uint8_t> flags(nq);
+    cuda_check(cudaMemcpyAsync(flags.data(), dflags, nq, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+    cuda_check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+    std::vector<uint32_t> redo;
+    for (uint64_t i = 0; i < nq; i++)
+        if (flags[i]) redo.push_back((uint32_t)i);
+    if (!redo.empty()) redo_exact(h, dq, redo, k, dallow, dl, dd, dc, st, false);
+    return true;
+}
+
+// Exact brute force of a batch on device buffers; may_sync: the caller waits
+// for the result anyway (the tensor-core route reads back which queries it
+// certified, so calls that only enqueue work keep the float32 kernels).
+static void run_bf_exact(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, const uint8_t* dallow,
+                         uint64_t* dl, float* dd, int32_t* dc, cudaStream_t st, bool may_sync) {
+    if (may_sync && bf_tensor_exact(h->count, nq, k, h->dim) && run_bf_certified(h, dq, nq, k, dallow, dl, dd, dc, st))
+        return;
+    run_bf_simt(h, dq, nq, k, dallow, dl, dd, dc, st);
+}
+
+// Exact answers of the queries listed in `redo`, in place; waits for them.
+static void redo_exact(hnswgpu_index* h, const float* dq, const std::vector<uint32_t>& redo, uint64_t k,
+                       const uint8_t* dallow, uint64_t* dl, float* dd, int32_t* dc, cudaStream_t st, bool tensor) {
+    const uint64_t m = redo.size(), dim = h->dim;
+    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t ib = al(m * 4), qb = al(m * dim * 4), lb = al(m * k * 8), db = al(m * k * 4);
+    PoolBuf ws(st);
+    cuda_check(ws.alloc(h, ib + qb + lb + db + m * 4), "exact scan workspace");
+    unsigned char* base = static_cast<unsigned char*>(ws.p);
+    uint32_t* idx = (uint32_t*)base;
+    float* rq = (float*)(base + ib);
+    uint64_t* rl = (uint64_t*)(base + ib + qb);
+    float* rd = (float*)(base + ib + qb + lb);
+    int32_t* rc = (int32_t*)(base + ib + qb + lb + db);
+    cuda_check(cudaMemcpyAsync(idx, redo.data(), m * 4, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
+    cuda_check(hnswgpu::launch_tc_gather(dq, idx, (uint32_t)m, (uint32_t)dim, rq, st), "gather launch");
+    run_bf_exact(h, rq, m, k, dallow, rl, rd, rc, st, tensor);
+    cuda_check(hnswgpu::launch_tc_scatter(idx, (uint32_t)m, (uint32_t)k, rl, rd, rc, dl, dd, dc, st), "scatter launch");
+    cuda_check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+}
+
 // Tensor-core brute force (bf_tc.cu) of a BruteforceSearch index over its
 // bf16 / fp8 copy: sampled threshold, tcgen05 scores with fused candidate
 // filtering, selection of the R best and exact float32 re-rank; queries the
@@ -768,16 +968,7 @@ void run_bf_tc(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint3
     const uint64_t R = std::max<uint64_t>(k, rerank ? rerank : 4 * k);
     if (R > 1024) throw ApiError(HNSWGPU_ERR_UNSUPPORTED, "tensor-core brute force: over-fetch (rerank, or 4 k) must be <= 1024");
     if (nq > 0x7fffffffull) throw ApiError(HNSWGPU_ERR_ARG, "batch too large");
-    const bool first = !h->tc_rowinfo[prec].p;
-    ensure_traversal_copy(h, prec);
-    const uint32_t trow = hnswgpu::traversal_row_bytes(prec, dim);
-    if (first) {
-        h->tc_rowinfo[prec].alloc((n + 255) / 256 * 256);  // whole tiles: read by 2 KB bulk copies
-        cuda_check(hnswgpu::launch_tc_rowinfo(h->vecs.p, (uint32_t)n, dim, h->row_floats, h->tcopy[prec].p, trow, prec,
-                                              h->tc_rowinfo[prec].p, h->stream),
-                   "rowinfo launch");
-        cuda_check(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
-    }
+    const uint32_t trow = ensure_tc_copy(h, prec);
     // sampling: about 5 R rows of the whole set below the 16th-best sampled distance
     const bool sampled = n > 16384;
     uint64_t step = 1, n_sample = n, cap = n;
@@ -802,7 +993,7 @@ void run_bf_tc(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint3
     h->tc_flags.ensure(nq);
     h->tc_buf.ensure(nq * cap);
     cuda_check(hnswgpu::launch_tc_query_prep(dq, (uint32_t)nq, dim, h->space == HNSWGPU_SPACE_COSINE, prec, trow,
-                                             h->tc_qf.p, h->tc_qt.p, h->tc_qscale.p, st),
+                                             h->tc_qf.p, h->tc_qt.p, h->tc_qscale.p, nullptr, 0, nullptr, st),
                "query prep launch");
     CUtensorMap qmap, xmap, smap;
     cuda_check(hnswgpu::tc_encode_map(h->tc_qt.p, prec, nq, dim, trow, 128, &qmap), "tensor map (queries)");
@@ -883,20 +1074,7 @@ void run_bf_tc(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint3
     for (uint64_t i = 0; i < nq; i++)
         if (flags[i]) redo.push_back((uint32_t)i);
     if (!redo.empty()) {
-        const uint64_t m = redo.size();
-        h->tc_idx.ensure(m);
-        DevBuf<float> rq, rd;
-        DevBuf<uint64_t> rl;
-        DevBuf<int32_t> rc;
-        rq.alloc(m * dim);
-        rd.alloc(m * k);
-        rl.alloc(m * k);
-        rc.alloc(m);
-        cuda_check(cudaMemcpyAsync(h->tc_idx.p, redo.data(), m * 4, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
-        cuda_check(hnswgpu::launch_tc_gather(dq, h->tc_idx.p, (uint32_t)m, dim, rq.p, st), "gather launch");
-        run_bf_exact(h, rq.p, m, k, dallow, rl.p, rd.p, rc.p, st);
-        cuda_check(hnswgpu::launch_tc_scatter(h->tc_idx.p, (uint32_t)m, (uint32_t)k, rl.p, rd.p, rc.p, dl, dd, dc, st),
-                   "scatter launch");
+        redo_exact(h, dq, redo, k, dallow, dl, dd, dc, st, true);
         if (dtrace) {
             // mark fallback queries in trace[2]
             std::vector<uint32_t> tr(nq * 4);
@@ -911,7 +1089,7 @@ void run_bf_tc(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint3
 
 void run_search(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint64_t ef, const uint8_t* dallow,
                 uint64_t* dl, float* dd, int32_t* dc, uint32_t* dtrace, cudaStream_t st, bool exact,
-                uint32_t prec, uint32_t rerank, const TermCfg* term, bool scan, bool replay_all) {
+                uint32_t prec, uint32_t rerank, const TermCfg* term, bool scan, bool replay_all, bool may_sync) {
     if (scan && !h->is_bf && h->num_deleted) {
         // deleted elements are never returned: fold them into the row mask
         h->scan_mask.ensure(h->count);
@@ -921,7 +1099,7 @@ void run_search(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint
     if (h->is_bf && prec) {
         run_bf_tc(h, dq, nq, k, rerank, dallow, dl, dd, dc, dtrace, st, prec);
     } else if (h->is_bf || scan) {
-        run_bf_exact(h, dq, nq, k, dallow, dl, dd, dc, st);
+        run_bf_exact(h, dq, nq, k, dallow, dl, dd, dc, st, may_sync);
     } else {
         run_hnsw(h, dq, nq, k, ef, dallow, dl, dd, dc, dtrace, st, exact, prec, rerank, term, replay_all);
     }
@@ -1240,7 +1418,7 @@ int hnswgpu_search(hnswgpu_index* h, const float* queries, uint64_t nq, uint64_t
         }
         cuda_check(cudaMemcpyAsync(dq, queries, qb, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
         run_search(h, dq, nq, k, ef, dallow, dl, dd, dc, dt, st, exact, o.precision, o.rerank, &term, scan,
-                   replay_all);
+                   replay_all, true);
         cuda_check(cudaMemcpyAsync(out_labels, dl, lb, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
         cuda_check(cudaMemcpyAsync(out_dists, dd, db, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
         cuda_check(cudaMemcpyAsync(out_counts, dc, cb, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");

@@ -104,8 +104,9 @@ struct hnswgpu_index {
     // tensor-core brute force: per-call workspace
     DevBuf<float> tc_qf, tc_qscale, tc_tau, tc_part;
     DevBuf<float2> tc_sinfo;           // helpers of the sampled rows
+    DevBuf<uint32_t> tc_stats;         // bf16 copy: largest row norm and rounding error norm (float bits)
     DevBuf<unsigned char> tc_qt;
-    DevBuf<uint32_t> tc_cnt, tc_idx;
+    DevBuf<uint32_t> tc_cnt;
     DevBuf<uint64_t> tc_buf;
     DevBuf<uint8_t> tc_flags;
     DevBuf<uint8_t> scan_mask;         // exact scan over an index with deletions
@@ -174,6 +175,6 @@ hnswgpu::SearchParams hnsw_params(const hnswgpu_index* h, const float* dq, uint6
 void run_search(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint64_t ef, const uint8_t* dallow,
                 uint64_t* dl, float* dd, int32_t* dc, uint32_t* dtrace, cudaStream_t st, bool exact,
                 uint32_t prec = 0, uint32_t rerank = 0, const TermCfg* term = nullptr, bool scan = false,
-                bool replay_all = false);
+                bool replay_all = false, bool may_sync = false);
 
 }  // namespace hnswgpu_host

@@ -111,3 +111,39 @@ def test_lists_that_overflow(prec):
         redo = tr[:, 2] == 1
         assert redo.any()
         assert np.array_equal(l[redo], el[redo]) and np.array_equal(d[redo], ed[redo])
+
+
+def _clusters(rng, n, dim, sigma):
+    c = rng.standard_normal((max(4, n // 500), dim)).astype(np.float32)
+    return (c[rng.integers(0, len(c), n)] + sigma * rng.standard_normal((n, dim))).astype(np.float32)
+
+
+@pytest.mark.parametrize("space", ["l2", "ip", "cosine"])
+@pytest.mark.parametrize("dim", [33, 100, 128])
+@pytest.mark.parametrize("sigma", [0.02, 0.5, 30.0])
+def test_certified_scan(tmp_path, space, dim, sigma):
+    """Batches large enough for the tensor-core route of the exact scan: tight
+    clusters (distances far below the scores' error), loose ones, and rows
+    whose norms differ; k on both sides of its sample sizes; a mask."""
+    rng = np.random.default_rng(dim)
+    x = _clusters(rng, 20000, dim, sigma)
+    x[::1000] *= 20.0
+    g, o = _pair(tmp_path, x, space)
+    q = _clusters(rng, 700, dim, sigma)
+    q[::2] = x[rng.integers(0, 20000, 350)] + np.float32(0.01)
+    for k in (1, 100, 101, 256):
+        _same(g, o, q, k)
+    _same(g, o, q, 10, filt=lambda v: v % 127 != 0 and v % 3 == 0)
+    _same(g, o, q, 10, filt=lambda v: v % 2000 == 5)
+
+
+def test_certified_scan_ties_and_range(tmp_path):
+    rng = np.random.default_rng(11)
+    x = rng.integers(0, 2, (30000, 40)).astype(np.float32)
+    x[10000:] = x[:20000]  # every distance at least twice
+    g, o = _pair(tmp_path, x, "l2")
+    q = rng.integers(0, 2, (600, 40)).astype(np.float32)
+    _same(g, o, q, 10)
+    for scale in (1e-21, 3e18):  # squares under- and overflow float32
+        g, o = _pair(tmp_path, x * np.float32(scale), "l2")
+        _same(g, o, q * np.float32(scale), 10)
