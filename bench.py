@@ -278,7 +278,7 @@ def recall(found, gt):
 class DeviceLoop:
     """Device-resident batch search through the C ABI (HNSWGPU_DEVICE_PTRS):
     queries and outputs stay in HBM; one kernel launch per step (two for the
-    reference tie order, whose two-pass search lists then replays)."""
+    reference tie order, which repeats some queries with the heaps)."""
 
     def __init__(self, idx, q, dev, k=10):
         import torch
@@ -513,8 +513,8 @@ def run_ours(args, dist: Dist):
         plain[order] = {"ef": ef_p, "recall@10": round(recall(lab_p, gt), 5), "ms_per_step": round(ms_p, 4),
                         "qps": round(dist.world * nq / (ms_p / 1e3), 1), "sweep": sw}
         if order == "reference":
-            # the same results by the one-pass heap replay of every query (the
-            # default replays only the queries whose id-order run met a tie)
+            # the same results by the heap replay of every query (the default
+            # replays only the queries whose id-order run met a tie that matters)
             o = loop.opts(ef_p, fl_p | _capi.REPLAY_ALL)
             loop.step(o)
             same = bool(np.array_equal(loop.labels(), lab_p))

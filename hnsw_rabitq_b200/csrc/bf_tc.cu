@@ -1085,9 +1085,8 @@ cudaError_t launch_fp64_distances(const float* q, uint64_t nq, uint32_t m, uint3
     return cudaGetLastError();
 }
 
-cudaError_t tc_encode_map(void* base, uint32_t prec, uint64_t rows, uint32_t dim, uint64_t row_pitch_bytes,
-                          uint32_t box_rows, CUtensorMap* out) {
-    // the driver entry point, looked up once (host threads may race here)
+// The driver entry point, looked up once (host threads may race here).
+static cudaError_t encode_entry(PFN_cuTensorMapEncodeTiled* out) {
     static std::atomic<PFN_cuTensorMapEncodeTiled> encode_fn{nullptr};
     PFN_cuTensorMapEncodeTiled encode = encode_fn.load(std::memory_order_acquire);
     if (!encode) {
@@ -1099,6 +1098,29 @@ cudaError_t tc_encode_map(void* base, uint32_t prec, uint64_t rows, uint32_t dim
         encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(fp);
         encode_fn.store(encode, std::memory_order_release);
     }
+    *out = encode;
+    return cudaSuccess;
+}
+
+cudaError_t gather_map(const void* base, uint64_t rows, uint32_t row_bytes, uint32_t slot_bytes, CUtensorMap* out) {
+    PFN_cuTensorMapEncodeTiled encode = nullptr;
+    cudaError_t e = encode_entry(&encode);
+    if (e != cudaSuccess) return e;
+    const cuuint64_t gdim[2] = {row_bytes / 4, rows};
+    const cuuint64_t gstride[1] = {row_bytes};
+    const cuuint32_t box[2] = {slot_bytes / 4, 1};
+    const cuuint32_t estride[2] = {1, 1};
+    CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), gdim, gstride, box, estride,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+cudaError_t tc_encode_map(void* base, uint32_t prec, uint64_t rows, uint32_t dim, uint64_t row_pitch_bytes,
+                          uint32_t box_rows, CUtensorMap* out) {
+    PFN_cuTensorMapEncodeTiled encode = nullptr;
+    cudaError_t e = encode_entry(&encode);
+    if (e != cudaSuccess) return e;
     const cuuint64_t gdim[2] = {dim, rows};
     const cuuint64_t gstride[1] = {row_pitch_bytes};
     const cuuint32_t box[2] = {prec == 1 ? (cuuint32_t)(kKBytes / 2) : (cuuint32_t)kKBytes, box_rows};

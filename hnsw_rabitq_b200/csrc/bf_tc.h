@@ -72,6 +72,9 @@ cudaError_t launch_fp64_distances(const float* q, uint64_t nq, uint32_t m, uint3
 size_t tc_select_smem(uint32_t sort_cap, uint32_t dim, uint32_t R);
 cudaError_t tc_encode_map(void* base, uint32_t prec, uint64_t rows, uint32_t dim, uint64_t row_pitch_bytes,
                           uint32_t box_rows, CUtensorMap* out);
+// Rows of row_bytes bytes (a multiple of 16) as 32-bit words, for gathers of
+// four rows into slots of slot_bytes (at most 1024) each.
+cudaError_t gather_map(const void* base, uint64_t rows, uint32_t row_bytes, uint32_t slot_bytes, CUtensorMap* out);
 cudaError_t launch_tc_scores(const CUtensorMap& qm, const CUtensorMap& xm, const TcArgs& a, uint32_t prec, int space,
                              int mode, int num_sms, cudaStream_t st);
 cudaError_t launch_tc_rowinfo(const float* vecs, uint32_t count, uint32_t dim, uint32_t row_floats,

@@ -940,7 +940,7 @@ cudaError_t launch_lean_s(const SearchParams& p, int num_sms, cudaStream_t strea
 }  // namespace
 
 bool lean_eligible(const SearchParams& p) {
-    if (p.prec != 2 || !p.bare || p.exact || p.tie_list || p.eps_mode || !p.fast16) return false;
+    if (p.prec != 2 || !p.bare || p.exact || p.eps_mode || !p.fast16) return false;
     if (p.maxM0 == 0 || p.maxM0 > 64) return false;
     const uint32_t D = p.trow_bytes - 16;
     return D % 32 == 0 && (D <= 128 || D % 128 == 0);

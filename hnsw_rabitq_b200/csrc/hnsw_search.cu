@@ -61,7 +61,7 @@ struct WarpSmem {
     uint64_t* topheap;   // tie-exact mode: replay of top_candidates
     SplitHeap candheap;  // tie-exact mode: replay of candidate_set
     int cand_total;      // tie-exact mode: its capacity (shared + spill)
-    uint64_t* accbuf;    // tie-exact mode: accepted keys of one chunk, link order
+    uint64_t* accbuf;    // accepted keys of one chunk, link order
     uint64_t* evbuf;     // tie-exact mode: keys evicted from top_candidates
 };
 
@@ -81,35 +81,72 @@ __device__ __forceinline__ bool dbg_ok(bool cond, unsigned code, unsigned long l
     }
     return false;
 }
-__device__ __forceinline__ void mbar_complete_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.complete_tx.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
 #define DBG_OK(cond, code, a, b) dbg_ok((cond), (code), (unsigned long long)(a), (unsigned long long)(b))
 #else
 #define DBG_OK(cond, code, a, b) true
 #endif
 
-// Staging copy with the optional checks: dst must lie in this warp's staging
-// region [stage, pool), src inside [base, base + nrows * row_bytes).
-__device__ __forceinline__ void stage_copy(const SearchParams& p, const WarpSmem& s, void* dst, const void* base,
-                                           uint64_t row, uint64_t nrows, uint32_t row_bytes, unsigned code) {
-#ifdef HNSWGPU_BOUNDS_CHECK
-    const unsigned char* dp = static_cast<const unsigned char*>(dst);
-    const unsigned char* lo = reinterpret_cast<const unsigned char*>(s.stage);
-    const unsigned char* hi = reinterpret_cast<const unsigned char*>(s.pool);
-    const bool ok = DBG_OK(dp >= lo && dp + row_bytes <= hi && ((uintptr_t)dp & 15) == 0 && (row_bytes & 15) == 0,
-                           code, dp - lo, row_bytes) &&
-                    DBG_OK(row < nrows, code + 1, row, nrows);
-#else
-    const bool ok = true;
-#endif
-    if (ok) {
-        bulk_g2s(dst, static_cast<const unsigned char*>(base) + row * row_bytes, row_bytes, s.bar);
+// Where the rows of one staging batch come from: the float32 rows, or the
+// low-precision traversal copy.
+struct RowSrc {
+    const unsigned char* base;
+    uint32_t row_bytes;      // bytes per row in global memory
+    uint32_t stage_bytes;    // staging stride
+    uint32_t slots;          // rows per batch
+    const CUtensorMap* map;  // rows of at most 256 words a stride: gathered four at a time (else null)
+};
+
+template <int PREC>
+__device__ __forceinline__ RowSrc trav_src(const SearchParams& p) {
+    if (PREC == 0) return RowSrc{reinterpret_cast<const unsigned char*>(p.vecs), p.row_bytes, p.stage_stride * 4,
+                                 p.stage_slots, p.gather ? &p.vmap : nullptr};
+    return RowSrc{p.tvecs, p.trow_bytes, p.tstage_bytes, p.tslots, p.tgather ? &p.tmap : nullptr};
+}
+
+// Start copying n rows into the staging slots [0, n): row j is the node held
+// by lane first + j.  One TMA gather brings four rows (the columns past the row
+// pad the slot): a lane's copy instruction costs the warp about 50 cycles
+// whatever its size, so 20 rows of 512 bytes in L2 take 890 cycles by five
+// gathers and 1690 by a bulk copy each (cp.async by 16 bytes a lane: 1190).
+// Longer rows keep the bulk copy: at 3 KB the two are 7 % apart.
+__device__ __forceinline__ void copy_rows(const SearchParams& p, const WarpSmem& s, const RowSrc& r, uint32_t id,
+                                          int first, int n, int lane) {
+    const uint32_t dst = smem_u32(s.stage), bar = smem_u32(s.bar);
+    fence_proxy_async_smem();
+    const int ng = (n + 3) >> 2;
+    if (lane == 0) mbar_arrive_expect_tx(s.bar, r.map ? (uint32_t)ng * 4u * r.stage_bytes : (uint32_t)n * r.row_bytes);
+    __syncwarp();
+    if (r.map) {
+        uint32_t y[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) y[k] = __shfl_sync(FULL, id, (first + min(4 * lane + k, n - 1)) & 31);
+        if (lane < ng &&
+            DBG_OK((size_t)ng * 4 * r.stage_bytes <= (size_t)(reinterpret_cast<const unsigned char*>(s.pool) -
+                                                              reinterpret_cast<const unsigned char*>(s.stage)),
+                   10, ng, r.stage_bytes) &&
+            DBG_OK(y[0] < p.count && y[1] < p.count && y[2] < p.count && y[3] < p.count, 11, y[0], y[3]))
+            asm volatile(
+                "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], "
+                "[%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst + (uint32_t)lane * 4u * r.stage_bytes),
+                "l"(r.map), "r"(0), "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(bar)
+                : "memory");
     } else {
-#ifdef HNSWGPU_BOUNDS_CHECK
-        mbar_complete_tx(s.bar, row_bytes);
-#endif
+        const uint32_t node = __shfl_sync(FULL, id, (first + lane) & 31);
+        if (lane < n && DBG_OK(node < p.count, 12, node, lane))
+            bulk_g2s(reinterpret_cast<unsigned char*>(s.stage) + (size_t)lane * r.stage_bytes,
+                     r.base + (uint64_t)node * r.row_bytes, r.row_bytes, s.bar);
     }
+}
+// The copies started last have landed (bounded; false: gave up).
+__device__ __forceinline__ bool copies_done(const WarpSmem& s, uint32_t& phase) {
+    const bool ok = mbar_wait(s.bar, phase);
+    phase ^= 1u;
+    return __all_sync(FULL, ok);
+}
+
+__device__ __forceinline__ void prefetch_row(const RowSrc& r, uint32_t id) {
+    const unsigned char* x = r.base + (uint64_t)id * r.row_bytes;
+    for (uint32_t o = 0; o < r.row_bytes; o += 128) prefetch_l2(x + o);
 }
 
 __device__ __forceinline__ bool is_allowed(const SearchParams& p, uint32_t id) {
@@ -159,8 +196,8 @@ __device__ __forceinline__ int insert_pos(const uint64_t* a, int cnt, uint32_t d
 }
 
 // Remove the nev (<= 32) distinct keys ev[0..nev) (all present) from the
-// sorted array a[0, size), keeping the order of the rest.
-__device__ __forceinline__ void remove_keys(uint64_t* a, int& size, const uint64_t* ev, int nev, int lane) {
+// sorted array a[0, size), keeping the order of the rest; returns what is left.
+__device__ __noinline__ int remove_keys(uint64_t* a, int size, const uint64_t* ev, int nev, int lane) {
     int myidx = lane < nev ? lower_bound_key(a, size, ev[lane] & KEY_MASK) : 0x7fffffff;
     int minidx = myidx;
 #pragma unroll
@@ -180,7 +217,7 @@ __device__ __forceinline__ void remove_keys(uint64_t* a, int& size, const uint64
         if (have && !gone) a[i - before] = e;
         __syncwarp();
     }
-    size -= nev;
+    return size - nev;
 }
 
 // First unexpanded entry at index >= hint, or -1.  Updates hint.
@@ -254,24 +291,41 @@ __device__ __forceinline__ int merge_sorted(uint64_t* a, int& size, int cap, uns
     return mpos;
 }
 
-// Stage the rows of up to `cnt` nodes into stage slots [0, cnt): lane `slot`
-// ... the calling lane copies row `id` into slot `slot` when `mine`.
-__device__ __forceinline__ bool stage_rows(const SearchParams& p, WarpSmem& s, uint32_t& phase, bool mine,
-                                           uint32_t id, int slot, int cnt, int lane) {
-    if (cnt == 0) return true;
-    fence_proxy_async_smem();
+// merge_sorted() with the na accepted keys also in shared memory, padded with
+// ~0 to an even count: their counts are pairs of broadcast reads instead of a
+// shuffle per key.  `key` may carry EXP_BIT, the keys in `keys` do not.
+__device__ __forceinline__ int merge_keys(uint64_t* a, int& size, int cap, bool mine, uint64_t key, int pos,
+                                          const uint64_t* keys, int na, int lane) {
+    const ulonglong2* k2 = reinterpret_cast<const ulonglong2*>(keys);
+    const uint64_t kc = key & KEY_MASK;
+    const int mpos = (int)__reduce_min_sync(FULL, mine ? (unsigned)pos : 0x7fffffffu);
+    int rank = 0;
+    for (int t = 0; t < na; t += 2) {
+        const ulonglong2 v = k2[t >> 1];
+        rank += (v.x < kc) + (v.y < kc);
+    }
+    if (size > mpos) {
+        // move the entries [mpos, size) right, last chunk first
+        for (int base = mpos + ((size - mpos - 1) & ~31); base >= mpos; base -= 32) {
+            const int i = base + lane;
+            const bool have = i < size;
+            const uint64_t e = have ? a[i] : 0;
+            const uint64_t em = e & KEY_MASK;
+            int sh = 0;
+            for (int t = 0; t < na; t += 2) {
+                const ulonglong2 v = k2[t >> 1];
+                sh += (v.x < em) + (v.y < em);
+            }
+            __syncwarp();
+            if (have && i + sh < cap) a[i + sh] = e;
+            __syncwarp();
+        }
+    }
+    const int np = pos + rank;
+    if (mine && np < cap) a[np] = key;
     __syncwarp();
-    if (lane == 0) mbar_arrive_expect_tx(s.bar, (uint32_t)cnt * p.row_bytes);
-    __syncwarp();
-    if (mine) stage_copy(p, s, s.stage + (size_t)slot * p.stage_stride, p.vecs, id, p.count, p.row_bytes, 10);
-    bool ok = mbar_wait(s.bar, phase);
-    phase ^= 1u;
-    return __all_sync(FULL, ok);
-}
-
-template <int SPACE>
-__device__ __forceinline__ float stage_dist(const SearchParams& p, const WarpSmem& s, int slot) {
-    return distance<SPACE>(s.q, s.stage + (size_t)slot * p.stage_stride, (int)p.dim);
+    size = min(size + na, cap);
+    return mpos;
 }
 
 struct Counters {
@@ -305,79 +359,100 @@ struct PhaseClock {
 #define PT_MARK(i)
 #endif
 
-// Distances of `cnt` (<= 32) nodes held by lanes [0, cnt) (id per lane);
-// result returned in the owning lane.  False on a wait timeout.
-// Rows are staged `stage_slots` at a time.  For dim % 16 == 0 each group of
-// 4 lanes evaluates one staged row (8 rows per pass, group4_dist16); other
-// dimensions use one lane per row with the scalar-order routine.
+// Distances of the staged rows [0, n) (4 lanes per row, 8 rows per pass) into
+// the lanes [s0, s0 + n).  FAST16 (dim % 16 == 0): two passes run together, so
+// that the reductions and shared-memory reads of one overlap the other's and a
+// query chunk is read once for both.  (Query chunks held in registers spilled
+// here, and the spills went to L2: shared memory leaves little L1.)  Other
+// dimensions use the 4-lane form of each summation order.
+template <int SPACE>
+__device__ __forceinline__ void acc_chunk(const float4& q, const float4& x, float (&c)[4]) {
+    if (SPACE == 0) {
+        const float t0 = __fsub_rn(q.x, x.x), t1 = __fsub_rn(q.y, x.y), t2 = __fsub_rn(q.z, x.z), t3 = __fsub_rn(q.w, x.w);
+        c[0] = __fmaf_rn(t0, t0, c[0]);
+        c[1] = __fmaf_rn(t1, t1, c[1]);
+        c[2] = __fmaf_rn(t2, t2, c[2]);
+        c[3] = __fmaf_rn(t3, t3, c[3]);
+    } else {
+        c[0] = __fmaf_rn(q.x, x.x, c[0]);
+        c[1] = __fmaf_rn(q.y, x.y, c[1]);
+        c[2] = __fmaf_rn(q.z, x.z, c[2]);
+        c[3] = __fmaf_rn(q.w, x.w, c[3]);
+    }
+}
+
 template <int SPACE, bool FAST16>
-__device__ __forceinline__ bool lane_distances(const SearchParams& p, WarpSmem& s, uint32_t& phase, uint32_t id,
+__device__ __forceinline__ void batch_dist(const SearchParams& p, const WarpSmem& s, int n, int s0, int lane,
+                                           float& dc) {
+    const int a = lane & 3;
+    const int n16 = (int)(p.dim >> 4);
+    auto row_of = [&](int i) {
+        const int v = min(i, n - 1);
+        const float* x = s.stage + (size_t)v * p.stage_stride;
+        if (!DBG_OK(reinterpret_cast<const unsigned char*>(x) + p.row_bytes <=
+                        reinterpret_cast<const unsigned char*>(s.pool),
+                    50, (size_t)v * p.stage_stride * 4, n))
+            x = s.stage;
+        return x;
+    };
+    auto route = [&](float r, int g) {
+        const int t = lane - s0 - g;  // this lane's row within the pass
+        const float got = __shfl_sync(FULL, r, (t & 7) << 2);
+        if (t >= 0 && t < 8 && t + g < n) dc = got;
+    };
+    if (!FAST16) {
+        for (int g = 0; g < n; g += 8) route(group4_dist<SPACE>(s.q, row_of(g + (lane >> 2)), (int)p.dim, a), g);
+        return;
+    }
+    const float4* q4 = reinterpret_cast<const float4*>(s.q) + a;
+#pragma unroll 1
+    for (int g = 0; g < n; g += 16) {
+        const float4* x4 = reinterpret_cast<const float4*>(row_of(g + (lane >> 2))) + a;
+        const float4* y4 = reinterpret_cast<const float4*>(row_of(g + 8 + (lane >> 2))) + a;
+        float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+        for (int c = 0; c < n16; c++) {
+            const float4 qv = q4[4 * c];
+            acc_chunk<SPACE>(qv, x4[4 * c], c0);
+            acc_chunk<SPACE>(qv, y4[4 * c], c1);
+        }
+        const float r0 = group4_reduce<SPACE>(c0[0], c0[1], c0[2], c0[3]);
+        const float r1 = group4_reduce<SPACE>(c1[0], c1[1], c1[2], c1[3]);
+        route(r0, g);
+        route(r1, g + 8);
+    }
+}
+
+// Distances of `cnt` (<= 32) nodes held by lanes [0, cnt) (id per lane);
+// result returned in the owning lane.  False on a wait timeout.  Rows are
+// staged `stage_slots` at a time.
+template <int SPACE, bool FAST16>
+__device__ __forceinline__ bool lane_distances(const SearchParams& p, const WarpSmem& s, uint32_t& phase, uint32_t id,
                                                int cnt, int lane, float& d, PhaseClock& pc) {
     d = __int_as_float(0x7f800000);
-    for (int s0 = 0; s0 < cnt; s0 += (int)p.stage_slots) {
-        const int n = min((int)p.stage_slots, cnt - s0);
-        const bool mine = lane >= s0 && lane < s0 + n;
-        if (!stage_rows(p, s, phase, mine, id, lane - s0, n, lane)) return false;
+    const RowSrc rs = trav_src<0>(p);
+    for (int s0 = 0; s0 < cnt; s0 += (int)rs.slots) {
+        const int n = min((int)rs.slots, cnt - s0);
+        copy_rows(p, s, rs, id, s0, n, lane);
+        if (!copies_done(s, phase)) return false;
         PT_MARK(4);
-        if (FAST16) {
-            const int a = lane & 3;
-            for (int g = 0; g < n; g += 8) {
-                const int v = min(g + (lane >> 2), n - 1);
-                float r = group4_dist16<SPACE>(s.q, s.stage + (size_t)v * p.stage_stride, (int)(p.dim >> 4), a);
-                const int rel = lane - s0 - g;  // this lane's row within the pass
-                float got = __shfl_sync(FULL, r, (rel & 7) << 2);
-                if (rel >= 0 && rel < 8 && mine) d = got;
-            }
-        } else {
-            float dt = lane < n ? stage_dist<SPACE>(p, s, lane) : 0.f;
-            float got = __shfl_sync(FULL, dt, (lane - s0) & 31);
-            if (mine) d = got;
-        }
+        batch_dist<SPACE, FAST16>(p, s, n, s0, lane, d);
         PT_MARK(5);
     }
     return true;
 }
 
 // ------------------------------------------------------------------------
-// Pipelined level-0 beam for dim % 16 == 0 and maxM0 <= 32 (with deletes or a
-// filter in the id tie order only).  Same decisions as the general loop; the
-// difference is scheduling: as soon as the acceptance of the current
-// expansion is known, the next candidate is fixed (id tie order: the first
-// unexpanded of pool + accepted; tie-exact order: the candidate heap's top,
-// predicted whenever its distance is unique), and its link row, visited-cache
-// update and first TMA batch are issued before the pool merge / heap replay
-// of the current expansion, which then run under that memory latency.
-// Where the rows of one staging batch come from: the float32 rows, or the
-// low-precision traversal copy.
-struct RowSrc {
-    const unsigned char* base;
-    uint32_t row_bytes;    // bytes per row in global memory (= bytes copied)
-    uint32_t stage_bytes;  // staging stride
-    uint32_t slots;        // rows per batch
-};
-
-template <int PREC>
-__device__ __forceinline__ RowSrc trav_src(const SearchParams& p) {
-    if (PREC == 0) return RowSrc{reinterpret_cast<const unsigned char*>(p.vecs), p.row_bytes, p.stage_stride * 4,
-                                 p.stage_slots};
-    return RowSrc{p.tvecs, p.trow_bytes, p.tstage_bytes, p.tslots};
-}
-
-__device__ __forceinline__ bool stage_src(const SearchParams& p, WarpSmem& s, uint32_t& phase, const RowSrc& r,
-                                          bool mine, uint32_t id, int slot, int cnt, int lane) {
-    if (cnt == 0) return true;
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) mbar_arrive_expect_tx(s.bar, (uint32_t)cnt * r.row_bytes);
-    __syncwarp();
-    if (mine)
-        stage_copy(p, s, reinterpret_cast<unsigned char*>(s.stage) + (size_t)slot * r.stage_bytes, r.base, id,
-                   p.count, r.row_bytes, 20);
-    bool ok = mbar_wait(s.bar, phase);
-    phase ^= 1u;
-    return __all_sync(FULL, ok);
-}
-
+// Pipelined level-0 beam for maxM0 <= 64 (with deletes or a filter in the id
+// tie order only).  Same decisions as the general loop; the difference is
+// scheduling: as soon as the acceptance of the current expansion is known, the
+// next candidate is fixed (id tie order: the first unexpanded of pool +
+// accepted; tie-exact order with live heaps: the candidate heap's top,
+// predicted whenever its distance is unique), and its visited-cache update and
+// first TMA batch are issued before the pool merge / heap operations of the
+// current expansion, which then run under that memory latency.  The list of
+// the candidate after that is loaded a whole expansion ahead (it is the right
+// one unless a closer neighbour turns up), and its rows are pulled into L2.
 struct Fetch {
     uint32_t id;     // this lane's neighbour id (link order), or INVALID_ID
     bool fresh;      // evaluated now (missed in the visited cache)
@@ -388,15 +463,27 @@ struct Fetch {
     bool allowed;    // FILTER: this lane's neighbour may be returned (not deleted, passes the filter)
 };
 
+// A node's level-0 list, two links per lane (maxM0 <= 64).
+struct LinkRow {
+    uint32_t a, b;
+};
+__device__ __forceinline__ LinkRow load_links(const SearchParams& p, uint32_t node, int lane) {
+    const uint32_t* l = p.links0 + (size_t)node * p.maxM0;
+    LinkRow r;
+    r.a = lane < (int)p.maxM0 ? __ldg(l + lane) : INVALID_ID;
+    r.b = lane + 32 < (int)p.maxM0 ? __ldg(l + 32 + lane) : INVALID_ID;
+    return r;
+}
+
+// Take up to 32 links (one per lane): visited-cache update, then the first
+// batch of row copies.
 // FILTER: also read each fresh neighbour's delete bit and filter byte (used
 // only after the row gather, so their latency overlaps it) and never admit
 // `skip` (a disallowed entry point, never stored with its distance).
 template <int PREC, bool FILTER = false>
-__device__ __forceinline__ void fetch_links(const SearchParams& p, WarpSmem& s, uint32_t c, int lane, Fetch& f,
-                                            uint32_t skip = INVALID_ID) {
+__device__ __forceinline__ void fetch_rows(const SearchParams& p, WarpSmem& s, uint32_t id, int lane, Fetch& f,
+                                           uint32_t skip = INVALID_ID) {
     const RowSrc rs = trav_src<PREC>(p);
-    const uint32_t* lrow = p.links0 + (size_t)c * p.maxM0;
-    const uint32_t id = lane < (int)p.maxM0 ? __ldg(lrow + lane) : INVALID_ID;
     bool fresh = id != INVALID_ID && (!FILTER || id != skip);
     if (!p.links_unique) {
         unsigned peers = __match_any_sync(FULL, id);
@@ -417,15 +504,16 @@ __device__ __forceinline__ void fetch_links(const SearchParams& p, WarpSmem& s, 
     __syncwarp();
     f.cid2 = s.cbuf[lane];
     f.n0 = min((int)rs.slots, f.nnew);
-    if (f.n0 > 0) {
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_expect_tx(s.bar, (uint32_t)f.n0 * rs.row_bytes);
-        __syncwarp();
-        if (lane < f.n0)
-            stage_copy(p, s, reinterpret_cast<unsigned char*>(s.stage) + (size_t)lane * rs.stage_bytes, rs.base,
-                       f.cid2, p.count, rs.row_bytes, 30);
-    }
+    if (f.n0 > 0) copy_rows(p, s, rs, f.cid2, 0, f.n0, lane);
+    if (lane >= f.n0 && lane < f.nnew) prefetch_row(rs, f.cid2);  // rows of the later batches: into L2 meanwhile
+}
+
+// Start pulling the rows of a list that will probably be expanded soon into L2
+// (those the visited cache does not hold).
+template <int PREC>
+__device__ __forceinline__ void prefetch_rows(const SearchParams& p, const WarpSmem& s, uint32_t id) {
+    const RowSrc rs = trav_src<PREC>(p);
+    if (id != INVALID_ID && s.vis[vis_slot(id, p.log2_vis)] != id) prefetch_row(rs, id);
 }
 
 // Approximate distances from staged low-precision rows [0, n) into the
@@ -507,74 +595,20 @@ __device__ __forceinline__ void batch_dist_lowp(const SearchParams& p, const War
     }
 }
 
-// Distances of the staged rows [0, n) into the compacted lanes [s0, s0 + n).
-template <int SPACE>
-__device__ __forceinline__ void batch_dist(const SearchParams& p, const WarpSmem& s, const float4* qr, int n, int s0,
-                                           int lane, float& dc) {
-    const int a = lane & 3;
-    const int n16 = (int)(p.dim >> 4);
-    for (int g = 0; g < n; g += 8) {
-        const int v = min(g + (lane >> 2), n - 1);
-        const float4* x4 = reinterpret_cast<const float4*>(s.stage + (size_t)v * p.stage_stride);
-        if (!DBG_OK(reinterpret_cast<const unsigned char*>(x4) + p.row_bytes <=
-                        reinterpret_cast<const unsigned char*>(s.pool),
-                    50, (size_t)v * p.stage_stride * 4, n))
-            x4 = reinterpret_cast<const float4*>(s.stage);
-        float r;
-        if (n16 <= 8) {
-            // query chunks held in registers (qr[c] = this lane's float4 of chunk c)
-            float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                if (c < n16) {
-                    const float4 qv = qr[c], xv = x4[4 * c + a];
-                    if (SPACE == 0) {
-                        float t0 = __fsub_rn(qv.x, xv.x), t1 = __fsub_rn(qv.y, xv.y), t2 = __fsub_rn(qv.z, xv.z),
-                              t3 = __fsub_rn(qv.w, xv.w);
-                        c0 = __fmaf_rn(t0, t0, c0);
-                        c1 = __fmaf_rn(t1, t1, c1);
-                        c2 = __fmaf_rn(t2, t2, c2);
-                        c3 = __fmaf_rn(t3, t3, c3);
-                    } else {
-                        c0 = __fmaf_rn(qv.x, xv.x, c0);
-                        c1 = __fmaf_rn(qv.y, xv.y, c1);
-                        c2 = __fmaf_rn(qv.z, xv.z, c2);
-                        c3 = __fmaf_rn(qv.w, xv.w, c3);
-                    }
-                }
-            }
-            r = group4_reduce<SPACE>(c0, c1, c2, c3);
-        } else {
-            r = group4_dist16<SPACE>(s.q, reinterpret_cast<const float*>(x4), n16, a);
-        }
-        const int t = lane - s0 - g;  // compacted index of this lane within the pass
-        const float got = __shfl_sync(FULL, r, (t & 7) << 2);
-        if (t >= 0 && t < 8 && t + g < n) dc = got;
-    }
-}
-
 // Distances of all fresh neighbours of a fetched list; result in the owning
-// (link-order) lane.
-template <int SPACE, int PREC>
-__device__ __forceinline__ bool fetch_distances(const SearchParams& p, WarpSmem& s, uint32_t& phase, const Fetch& f,
-                                                const float4* qr, int lane, float& d, PhaseClock& pc) {
+// (link-order) lane.  `guess`: a link of the list most likely fetched next.
+template <int SPACE, bool FAST16, int PREC>
+__device__ __forceinline__ bool fetch_distances(const SearchParams& p, const WarpSmem& s, uint32_t& phase,
+                                                const Fetch& f, int lane, float& d, uint32_t guess, PhaseClock& pc) {
     float dc = __int_as_float(0x7f800000);
     const RowSrc rs = trav_src<PREC>(p);
-    if (f.n0 > 0) {
-        const bool ok = mbar_wait(s.bar, phase);
-        phase ^= 1u;
-        if (!__all_sync(FULL, ok)) return false;
-        PT_MARK(4);
-        if (PREC == 0) batch_dist<SPACE>(p, s, qr, f.n0, 0, lane, dc);
-        else batch_dist_lowp<SPACE, PREC>(p, s, f.n0, 0, lane, dc);
-        PT_MARK(5);
-    }
-    for (int s0 = f.n0; s0 < f.nnew; s0 += (int)rs.slots) {
+    for (int s0 = 0; s0 < f.nnew; s0 += (int)rs.slots) {
         const int n = min((int)rs.slots, f.nnew - s0);
-        const bool mine = lane >= s0 && lane < s0 + n;
-        if (!stage_src(p, s, phase, rs, mine, f.cid2, lane - s0, n, lane)) return false;
+        if (s0) copy_rows(p, s, rs, f.cid2, s0, n, lane);
+        if (!copies_done(s, phase)) return false;
         PT_MARK(4);
-        if (PREC == 0) batch_dist<SPACE>(p, s, qr, n, s0, lane, dc);
+        if (s0 == 0) prefetch_rows<PREC>(p, s, guess);  // (its list has arrived with the rows)
+        if (PREC == 0) batch_dist<SPACE, FAST16>(p, s, n, s0, lane, dc);
         else batch_dist_lowp<SPACE, PREC>(p, s, n, s0, lane, dc);
         PT_MARK(5);
     }
@@ -695,15 +729,69 @@ __device__ __forceinline__ void term_final_row(const SearchParams& p, const Warp
     if (lane == 0) p.ckpt_count[qi] = r + 1;
 }
 
-// TIES (id order only): flag the query (status kTieBit) when its run meets a
-// distance tie that can make the reference's heaps decide differently from the
-// (distance, id) order.  With acceptance by counting (independent of heap
-// layout), the two runs agree step by step unless (a) the candidate popped next
-// shares its distance with another unexpanded candidate, or (b) the entries
-// dropped from the full pool tie with its new worst entry (an evicted entry that
-// stays in candidate_set at lowerBound would still be expanded); (c), the
-// top-k boundary tie, is checked by the caller.
-//
+// The tie-exact order (EXACT) without heaps.  Acceptance is by counting and does
+// not depend on heap layout, so a run in the (distance, id) order and the
+// reference's run differ only where distances tie, and most ties cannot change
+// the outcome:
+//   (a) The candidate popped next shares its distance d with another one.  Both
+//       runs then expand the tied candidates and everything they find at d or
+//       closer, in different orders, before they go beyond d.  If lowerBound
+//       is still above d when that is done, every one of these nodes was
+//       accepted and expanded in either order: lowerBound only falls as nodes
+//       are seen, so it was above d all along.  The same nodes have been seen,
+//       the pools hold the same distances, and what one run accepted and the
+//       other rejected lies beyond lowerBound, where a candidate can only end
+//       the search.  (A neighbour rejected meanwhile at exactly lowerBound
+//       could be such a difference: it counts as a tie that matters.)
+//   (b) The entry dropped from the full pool ties with its new worst entry.
+//       The reference may keep the other one, and both stay in its
+//       candidate_set; that matters only if candidates at that distance come up
+//       for expansion (or the search ends) while lowerBound is still there.
+//   (c) The k-th and the next result tie: the heap's layout decides.
+// A query that meets a tie that can matter is run again with the reference's
+// heaps, operation by operation (LIVE), by the same warp.  On 1M x 128 integer
+// vectors at ef 50, 11 % of the queries meet a tie of the three kinds and far
+// fewer one that can matter.
+struct HeapState {
+    bool live = false;  // the run keeps the reference's heaps
+    int tsz = 1;        // top_candidates entries (the entry point at first)
+    int csz = 0;        // candidate_set entries
+};
+
+// Rare code out of line, with its arguments by value: inlined at each use it
+// cost the whole beam registers (spilled to L2 at full occupancy), and a
+// reference would keep the state in local memory.
+struct HeapSizes {
+    int csz, tsz, nev, ovf;
+};
+// The reference's heap operations for the na accepted keys in acc; the
+// evicted ones go to ev.
+__device__ __noinline__ HeapSizes replay_push(SplitHeap cand, int cand_total, uint64_t* top, const uint64_t* acc,
+                                              uint64_t* ev, int na, int ef, int csz, int tsz, int lane) {
+    int nev = 0, ovf = 0;
+    if (lane == 0) {
+        for (int t = 0; t < na; t++) {
+            const uint64_t e = acc[t];
+            if (csz < cand_total) ref_heap_push(cand, csz, e, CandLess());
+            else ovf = 1;
+            ref_heap_push(top, tsz, e, TopLess());
+            if (tsz > ef) ev[nev++] = ref_heap_pop(top, tsz, TopLess());
+        }
+    }
+    __syncwarp();
+    return HeapSizes{__shfl_sync(FULL, csz, 0), __shfl_sync(FULL, tsz, 0), __shfl_sync(FULL, nev, 0),
+                     __shfl_sync(FULL, ovf, 0)};
+}
+
+__device__ __forceinline__ int push_heaps(const SearchParams& p, const WarpSmem& s, int lane, int na, HeapState& h,
+                                          uint32_t& status) {
+    const HeapSizes z = replay_push(s.candheap, s.cand_total, s.topheap, s.accbuf, s.evbuf, na, (int)p.ef, h.csz, h.tsz, lane);
+    h.csz = z.csz;
+    h.tsz = z.tsz;
+    if (z.ovf) status |= HNSWGPU_STATUS_OVERFLOW_BIT;
+    return z.nev;
+}
+
 // FILTER (id order only): deletions and / or an allow mask, as in the
 // reference's non-bare-bone loop (hnswalg.h:330-440).  Accepted neighbours that
 // may not be returned go to the sorted list s.extra instead of the pool: they
@@ -712,39 +800,47 @@ __device__ __forceinline__ void term_final_row(const SearchParams& p, const Warp
 // is above lowerBound; list entries beyond lowerBound are dropped, since they
 // can only end the search.  A disallowed entry point (ep_ok false) is expanded
 // first and never stored.
-template <int SPACE, bool EXACT, int PREC, int TERM, bool TIES = false, bool FILTER = false>
-__device__ bool base_pipelined(const SearchParams& p, WarpSmem& s, uint32_t& phase, int lane, Counters& ct,
-                               PhaseClock& pc, const float4* qr, uint32_t ep, float d0, int& psize, int& tsz,
-                               uint32_t& status, uint32_t qi, float qn, bool ep_ok = true) {
+//
+// A list longer than 32 links (maxM0 <= 64) is taken in two units, the second
+// without a choice in between: the sequential acceptance test over the first 32
+// neighbours and then over the rest is the test over all of them.
+//
+// LIVE: the loop with the reference's heaps.  It is a loop of its own because
+// instruction fetch bounds these loops at full occupancy (with both forms in
+// one, 4.3 of 10 cycles an instruction went to instruction-cache misses); for
+// the same reason nothing in them is unrolled far and what is rare is out of
+// line.
+struct Beam {
+    Fetch f;             // the unit in flight
+    uint32_t rest;       // links of the node's second unit
+    LinkRow guess;       // the list of the node most likely expanded after the one in flight
+    uint32_t guess_id;
+    int hint_p;
+};
+enum { kBeamFailed = 0, kBeamDone = 1, kBeamTie = 2 };
+
+template <int SPACE, bool FAST16, bool EXACT, int PREC, int TERM, bool FILTER, bool LIVE>
+__device__ __forceinline__ int beam_loop(const SearchParams& p, WarpSmem& s, uint32_t& phase, int lane, Counters& ct,
+                                         PhaseClock& pc, Beam& b, float d0, int& psize, HeapState& hs,
+                                         uint32_t& status, uint32_t qi, float qn, uint32_t skip_id, TermState& ts) {
     const int ef = (int)p.ef;
     const int kq = (int)p.k;
-    TermState ts;
     const int pcap = (int)p.pool_cap;
-    int hint_p = 0, csz = 0;
     int xsize = 0, hint_x = 0;  // FILTER: the list of disallowed candidates
     const int xcap = (int)p.extra_cap;
-    const uint32_t skip_id = FILTER && !ep_ok ? ep : INVALID_ID;
-    // the entry point is pushed and popped at once (hnswalg.h:325-359)
-    if (lane == 0 && (!FILTER || ep_ok)) {
-        s.pool[0] = mkkey(d0, ep) | (EXACT ? 0u : EXP_BIT);
-        if (EXACT) s.topheap[0] = mkkey(d0, ep);
-    }
-    psize = !FILTER || ep_ok ? 1 : 0;
-    tsz = EXACT ? 1 : 0;
-    __syncwarp();
-    Fetch f;
-    fetch_links<PREC, FILTER>(p, s, ep, lane, f, skip_id);
-    ct.l0_exp += 1;
-    PT_MARK(3);
+    uint32_t tie_a = 0, tie_b = 0;  // EXACT: distances of the ties (a), (b) not settled yet (keys; 0: none)
     while (true) {
-        ct.l0_dists += f.nnew;
         float d;
-        if (!fetch_distances<SPACE, PREC>(p, s, phase, f, qr, lane, d, pc)) return false;
+        ct.l0_dists += b.f.nnew;
+        if (!fetch_distances<SPACE, FAST16, PREC>(p, s, phase, b.f, lane, d, LIVE ? INVALID_ID : b.guess.a, pc))
+            return kBeamFailed;
+        const Fetch& f = b.f;
         // ---- acceptance (closed form of hnswalg.h:395 over the link order)
         const uint32_t dk = fkey(d);
         const bool full = psize == ef;
         const uint32_t lbk = full ? khi(s.pool[psize - 1]) : 0xffffffffu;
         bool live = f.fresh && !(full && dk >= lbk);
+        bool matters = EXACT && !LIVE && tie_a && __any_sync(FULL, f.fresh && full && dk == lbk);
         uint64_t key = ((uint64_t)dk << 32) | f.id;
         int posP = 0, cntP = 0, posX = 0;
         if (live) {
@@ -756,13 +852,18 @@ __device__ bool base_pipelined(const SearchParams& p, WarpSmem& s, uint32_t& pha
         }
         const bool allowed = !FILTER || f.allowed;
         const unsigned amask = __ballot_sync(FULL, live && allowed);
+        const int nlive = __popc(amask);
+        bool accept = live;
         int cntN = 0;
-        for (unsigned m = amask; m; m &= m - 1) {
-            const int src2 = __ffs(m) - 1;
-            const uint32_t dk2 = __shfl_sync(FULL, dk, src2);
-            cntN += (src2 < lane && dk2 <= dk);
+        if (TERM || psize + nlive >= ef) {  // (else every live neighbour fits)
+            // earlier neighbours at most as far: their keys, compacted in link order
+            const int mine = __popc(amask & lanemask_lt());
+            __syncwarp();
+            if (live && allowed) s.cbuf[mine] = dk;
+            __syncwarp();
+            for (int t = 0; t < nlive; t++) cntN += (t < mine) & (s.cbuf[t] <= dk);
+            accept = live && cntP + cntN < ef;
         }
-        const bool accept = live && cntP + cntN < ef;
         const unsigned pmask = __ballot_sync(FULL, accept && allowed);
         const unsigned xmask = FILTER ? __ballot_sync(FULL, accept && !allowed) : 0u;
         if (TERM && __any_sync(FULL, accept && allowed && cntP + cntN < kq)) {
@@ -770,105 +871,115 @@ __device__ bool base_pipelined(const SearchParams& p, WarpSmem& s, uint32_t& pha
             ts.nchange++;
         }
         PT_MARK(6);
-        // ---- the next candidate
-        // smallest accepted key: the smallest distance key, then the smallest
-        // id among the lanes holding it (two warp reductions)
-        const uint32_t kmin_hi = __reduce_min_sync(FULL, accept ? dk : 0xffffffffu);
-        const uint32_t kmin_lo = __reduce_min_sync(FULL, accept && dk == kmin_hi ? f.id : 0xffffffffu);
-        const uint64_t kmin = ((uint64_t)kmin_hi << 32) | kmin_lo;
-        bool have_next = false, spec = false, next_extra = false;
+        // ---- the next unit: the rest of this list, or the next candidate
+        bool inner = __any_sync(FULL, b.rest != INVALID_ID);
+        bool have_next = inner, spec = false, next_extra = false;
         uint32_t next = INVALID_ID, next_dk = 0xffffffffu;
-        if (!EXACT) {
-            int ip = find_unexpanded(s.pool, psize, hint_p, lane);
-            const uint64_t kp = ip >= 0 ? (s.pool[ip] & KEY_MASK) : ~0ull;
-            int ix = -1;
-            uint64_t kx = ~0ull;
-            if (FILTER) {
-                ix = find_unexpanded(s.extra, xsize, hint_x, lane);
-                kx = ix >= 0 ? (s.extra[ix] & KEY_MASK) : ~0ull;
-            }
-            if (kx < kp && kx < kmin) {
-                // a disallowed candidate from the list (FILTER only)
-                have_next = true;
-                next_extra = true;
-                next_dk = khi(kx);
-                next = kid(kx);
-                __syncwarp();
-                if (lane == 0) s.extra[ix] |= EXP_BIT;
-                __syncwarp();
-            } else if (kp != ~0ull || kmin != ~0ull) {
-                have_next = true;
-                next_dk = khi(kmin < kp ? kmin : kp);
-                if (TIES) {  // (a): candidate_set's top must be unique by distance
-                    int same = __popc(__ballot_sync(FULL, accept && dk == next_dk));
-                    if (ip >= 0) same += unexpanded_with_dist(s.pool, psize, ip, next_dk, lane);
-                    if (same > 1) status |= kTieBit;
-                }
-                if (kmin < kp) {
-                    next = (uint32_t)kmin;
-                    if (FILTER) next_extra = __any_sync(FULL, accept && !allowed && key == kmin);
-                    if (accept && key == kmin) key |= EXP_BIT;  // inserted already expanded
-                } else {
-                    next = kid(kp);
-                    __syncwarp();
-                    if (lane == 0) s.pool[ip] |= EXP_BIT;
-                    __syncwarp();
-                }
-            }
-        } else {
-            // candidate_set after this expansion's pushes: its top is the
-            // smallest of the current heap top and the accepted keys; when
-            // that distance is unique the heap layout cannot matter
-            const uint64_t r0 = csz > 0 ? s.candheap[0] : ~0ull;
-            const uint32_t r0d = khi(r0);
-            const bool r0tie = (csz > 1 && khi(s.candheap[1]) == r0d) || (csz > 2 && khi(s.candheap[2]) == r0d);
-            const uint32_t ad = khi(kmin);
-            const uint32_t nd = min(r0d, ad);
-            const int acount = __popc(__ballot_sync(FULL, accept && dk == nd));
-            const int mult = (csz > 0 && r0d == nd ? 1 + (r0tie ? 1 : 0) : 0) + acount;
-            if ((csz > 0 || kmin != ~0ull) && mult == 1) {
-                spec = true;
-                next = r0d == nd && csz > 0 ? kid(r0) : (uint32_t)kmin;
-            }
-        }
         Fetch fn;
-        if (have_next || spec) fetch_links<PREC, FILTER>(p, s, next, lane, fn, skip_id);
-        PT_MARK(2);
-        // ---- bookkeeping of this expansion, under the latency of the next fetch
-        int nev = 0;
-        if (EXACT && pmask) {
-            if (accept) s.accbuf[__popc(pmask & lanemask_lt())] = key;
-            __syncwarp();
-            const int na = __popc(pmask);
-            uint32_t ovf = 0;
-            if (lane == 0) {
-                int cn = csz, tn = tsz;
-                for (int t = 0; t < na; t++) {
-                    const uint64_t e = s.accbuf[t];
-                    if (cn < s.cand_total) ref_heap_push(s.candheap, cn, e, CandLess());
-                    else ovf = 1;
-                    ref_heap_push(s.topheap, tn, e, TopLess());
-                    if (tn > ef) s.evbuf[nev++] = ref_heap_pop(s.topheap, tn, TopLess());
+        {
+            if (!inner) {
+                // smallest accepted key: the smallest distance key, then the smallest
+                // id among the lanes holding it (two warp reductions)
+                const uint32_t kmin_hi = __reduce_min_sync(FULL, accept ? dk : 0xffffffffu);
+                const uint32_t kmin_lo = __reduce_min_sync(FULL, accept && dk == kmin_hi ? f.id : 0xffffffffu);
+                const uint64_t kmin = ((uint64_t)kmin_hi << 32) | kmin_lo;
+                if (LIVE) {
+                    // candidate_set after this expansion's pushes: its top is the
+                    // smallest of the current heap top and the accepted keys; when
+                    // that distance is unique the heap layout cannot matter
+                    const uint64_t r0 = hs.csz > 0 ? s.candheap[0] : ~0ull;
+                    const uint32_t r0d = khi(r0);
+                    const bool r0tie = (hs.csz > 1 && khi(s.candheap[1]) == r0d) || (hs.csz > 2 && khi(s.candheap[2]) == r0d);
+                    const uint32_t nd = min(r0d, kmin_hi);
+                    const int acount = __popc(__ballot_sync(FULL, accept && dk == nd));
+                    const int mult = (hs.csz > 0 && r0d == nd ? 1 + (r0tie ? 1 : 0) : 0) + acount;
+                    if ((hs.csz > 0 || kmin != ~0ull) && mult == 1) {
+                        spec = true;
+                        next = r0d == nd && hs.csz > 0 ? kid(r0) : (uint32_t)kmin;
+                    }
+                } else {
+                    int ip = find_unexpanded(s.pool, psize, b.hint_p, lane);
+                    const uint64_t kp = ip >= 0 ? (s.pool[ip] & KEY_MASK) : ~0ull;
+                    int ix = -1;
+                    uint64_t kx = ~0ull;
+                    if (FILTER) {
+                        ix = find_unexpanded(s.extra, xsize, hint_x, lane);
+                        kx = ix >= 0 ? (s.extra[ix] & KEY_MASK) : ~0ull;
+                    }
+                    if (kx < kp && kx < kmin) {
+                        // a disallowed candidate from the list (FILTER only)
+                        have_next = true;
+                        next_extra = true;
+                        next_dk = khi(kx);
+                        next = kid(kx);
+                        __syncwarp();
+                        if (lane == 0) s.extra[ix] |= EXP_BIT;
+                        __syncwarp();
+                    } else if (kp != ~0ull || kmin != ~0ull) {
+                        have_next = true;
+                        next_dk = khi(kmin < kp ? kmin : kp);
+                        if (EXACT) {  // (a): candidate_set's top must be unique by distance
+                            int same = __popc(__ballot_sync(FULL, accept && dk == next_dk));
+                            if (ip >= 0) same += unexpanded_with_dist(s.pool, psize, ip, next_dk, lane);
+                            if (same > 1) tie_a = max(tie_a, next_dk);
+                        }
+                        if (kmin < kp) {
+                            next = (uint32_t)kmin;
+                            if (FILTER) next_extra = __any_sync(FULL, accept && !allowed && key == kmin);
+                            if (accept && key == kmin) key |= EXP_BIT;  // inserted already expanded
+                        } else {
+                            next = kid(kp);
+                            __syncwarp();
+                            if (lane == 0) s.pool[ip] |= EXP_BIT;
+                            __syncwarp();
+                        }
+                    }
                 }
-                csz = cn;
-                tsz = tn;
             }
-            csz = __shfl_sync(FULL, csz, 0);
-            tsz = __shfl_sync(FULL, tsz, 0);
-            nev = __shfl_sync(FULL, nev, 0);
-            if (__shfl_sync(FULL, ovf, 0)) status |= HNSWGPU_STATUS_OVERFLOW_BIT;
-            __syncwarp();
-            PT_MARK(7);
+            if (have_next || spec) {
+                LinkRow row{b.rest, INVALID_ID};
+                if (!inner) row = !LIVE && next == b.guess_id ? b.guess : load_links(p, next, lane);
+                b.rest = row.b;
+                fetch_rows<PREC, FILTER>(p, s, row.a, lane, fn, skip_id);
+                prefetch_rows<PREC>(p, s, row.b);  // (none but in a list of more than 32 links)
+            }
         }
-        if (pmask) {
-            const int m = merge_sorted(s.pool, psize, pcap, pmask, key, posP, lane);
-            hint_p = min(hint_p, m);
-            if (TIES && psize > ef) {
-                // (b): the merge kept one entry more than ef (pool_cap is
-                // ef + 1): the first one dropped, next to the new worst
-                if (khi(s.pool[ef]) == khi(s.pool[ef - 1])) status |= kTieBit;
+        PT_MARK(2);
+        // ---- bookkeeping of this unit, under the latency of the next fetch
+        const int na = __popc(pmask);
+        if (na) {
+            // the accepted keys in link order, padded to an even count
+            const bool put = accept && allowed;
+            if (put) s.accbuf[__popc(pmask & lanemask_lt())] = key & KEY_MASK;
+            else if ((na & 1) && lane == __ffs(~pmask) - 1) s.accbuf[na] = ~0ull;
+            __syncwarp();
+            int nev = 0;
+            if (LIVE) {
+                nev = push_heaps(p, s, lane, na, hs, status);
+                PT_MARK(7);
+            }
+            const int m = merge_keys(s.pool, psize, pcap, put, key, posP, s.accbuf, na, lane);
+            b.hint_p = min(b.hint_p, m);
+            if (EXACT && !LIVE && psize > ef) {
+                if (khi(s.pool[ef]) == khi(s.pool[ef - 1])) tie_b = khi(s.pool[ef]);
                 psize = ef;
             }
+            if (LIVE && nev) psize = remove_keys(s.pool, psize, s.evbuf, nev, lane);
+        }
+        if (EXACT && !LIVE && (tie_a | tie_b) && !inner) {
+            // settle the open ties against lowerBound after this expansion
+            const uint32_t lb = psize == ef ? khi(s.pool[ef - 1]) : 0xffffffffu;
+            const uint32_t nd = have_next ? next_dk : 0xffffffffu;
+            if (tie_a && nd > tie_a) {
+                matters |= lb <= tie_a;
+                tie_a = 0;
+            }
+            if (lb < tie_b) tie_b = 0;
+            matters |= tie_b && nd >= tie_b;
+        }
+        if (EXACT && !LIVE && matters) {
+            if (have_next && fn.n0 > 0) copies_done(s, phase);
+            return kBeamTie;
         }
         if (FILTER) {
             if (xmask) {
@@ -881,98 +992,138 @@ __device__ bool base_pipelined(const SearchParams& p, WarpSmem& s, uint32_t& pha
                 xsize = upper_bound_hi(s.extra, xsize, khi(s.pool[psize - 1]));
                 hint_x = min(hint_x, xsize);
             }
-            if (next_extra && psize == ef && next_dk > khi(s.pool[ef - 1])) {
-                // the reference pops it and stops (hnswalg.h:345-347): drain
-                // the speculative fetch
-                if (fn.n0 > 0) {
-                    mbar_wait(s.bar, phase);
-                    phase ^= 1u;
-                }
-                break;
-            }
-            if (have_next && ct.l0_exp >= p.max_expansions) {
+            bool stop = next_extra && psize == ef && next_dk > khi(s.pool[ef - 1]);
+            if (have_next && !inner && !stop && ct.l0_exp >= p.max_expansions) {
                 // Entries dropped from a full list can be re-admitted after a
                 // visited-cache miss, and a search that never fills its pool
                 // (a filter that rejects almost everything) keeps dropping
                 // them: bound the expansions and flag the query.
                 status |= HNSWGPU_STATUS_OVERFLOW_BIT;
-                if (fn.n0 > 0) {
-                    mbar_wait(s.bar, phase);
-                    phase ^= 1u;
-                }
-                break;
+                stop = true;
+            }
+            if (stop) {
+                // the reference pops it and stops (hnswalg.h:345-347): drain
+                // the speculative fetch
+                if (fn.n0 > 0) copies_done(s, phase);
+                return kBeamDone;
             }
         }
-        if (EXACT && nev) remove_keys(s.pool, psize, s.evbuf, nev, lane);
-        if (!EXACT) {
+        if (!LIVE && !inner) {
             // the expansion after `next` is most often the first unexpanded
-            // entry now: pull its link row into L2 while `next` runs
-            int h2 = hint_p;
+            // entry now: load its list while `next` runs
+            int h2 = b.hint_p;
             const int nx = find_unexpanded(s.pool, psize, h2, lane);
-            if (nx >= 0 && lane == 0) prefetch_l2(p.links0 + (size_t)kid(s.pool[nx]) * p.maxM0);
+            if (nx >= 0) {
+                b.guess_id = kid(s.pool[nx]);
+                b.guess = load_links(p, b.guess_id, lane);
+            }
         }
         PT_MARK(8);
-        if (TIES && (status & kTieBit)) {
-            // listed for the heap replay, which recomputes the whole query:
-            // drain the prefetched expansion and stop here
-            if (have_next && fn.n0 > 0) {
-                mbar_wait(s.bar, phase);
-                phase ^= 1u;
-            }
-            break;
-        }
-        if (TERM && have_next && term_due(p, s, ct.l0_exp, psize, next_dk, ts) &&
+        if (TERM && have_next && !inner && term_due(p, s, ct.l0_exp, psize, next_dk, ts) &&
             term_checkpoint<SPACE, TERM>(p, s, lane, qi, ct.l0_exp, ct.l0_dists, psize, next_dk, d0, qn, ts)) {
             // confident that the top-k is final: drain the prefetched
             // expansion and stop
-            if (fn.n0 > 0) {
-                mbar_wait(s.bar, phase);
-                phase ^= 1u;
-            }
-            break;
+            if (fn.n0 > 0) copies_done(s, phase);
+            return kBeamDone;
         }
-        if (EXACT) {
-            // the reference's loop head: top of candidate_set vs lowerBound
-            bool go = false;
-            uint32_t top_id = INVALID_ID;
-            if (csz > 0) {
-                const uint64_t c = s.candheap[0];
-                const uint32_t lb = khi(s.pool[psize - 1]);
-                go = !(khi(c) > lb);
-                top_id = kid(c);
-            }
-            if (!go) {
-                if (spec && fn.n0 > 0) {  // drain the unused copies
-                    mbar_wait(s.bar, phase);
-                    phase ^= 1u;
+        if (!inner) {
+            if (LIVE) {
+                // the reference's loop head: top of candidate_set vs lowerBound
+                bool go = false;
+                uint32_t top_id = INVALID_ID;
+                if (hs.csz > 0) {
+                    const uint64_t c = s.candheap[0];
+                    const uint32_t lb = khi(s.pool[psize - 1]);
+                    go = !(khi(c) > lb);
+                    top_id = kid(c);
                 }
-                break;
-            }
-            __syncwarp();
-            if (lane == 0) {
-                int n = csz;
-                ref_heap_pop(s.candheap, n, CandLess());
-                if (n > 0) prefetch_l2(p.links0 + (size_t)kid(s.candheap[0]) * p.maxM0);
-            }
-            csz--;
-            __syncwarp();
-            if (spec && top_id != next) {
-                // only after a full candidate heap dropped a push (flagged as
-                // an overflow): fetch the actual top instead
-                if (fn.n0 > 0) {
-                    mbar_wait(s.bar, phase);
-                    phase ^= 1u;
+                if (!go) {
+                    if (spec && fn.n0 > 0) copies_done(s, phase);  // drain the unused copies
+                    return kBeamDone;
                 }
-                spec = false;
+                __syncwarp();
+                if (lane == 0) {
+                    int n = hs.csz;
+                    ref_heap_pop(s.candheap, n, CandLess());
+                    if (n > 0) prefetch_l2(p.links0 + (size_t)kid(s.candheap[0]) * p.maxM0);
+                }
+                hs.csz--;
+                __syncwarp();
+                if (spec && top_id != next) {
+                    // only after a full candidate heap dropped a push (flagged as
+                    // an overflow): fetch the actual top instead
+                    if (fn.n0 > 0) copies_done(s, phase);
+                    spec = false;
+                }
+                if (!spec) {
+                    const LinkRow row = load_links(p, top_id, lane);
+                    b.rest = row.b;
+                    fetch_rows<PREC>(p, s, row.a, lane, fn);
+                }
+            } else if (!have_next) {
+                return kBeamDone;
             }
-            if (!spec) fetch_links<PREC>(p, s, top_id, lane, fn);
-        } else if (!have_next) {
-            break;
+            ct.l0_exp += 1;
         }
-        f = fn;
-        ct.l0_exp += 1;
+        b.f = fn;
         PT_MARK(2);
     }
+}
+
+template <int SPACE, bool FAST16, bool EXACT, int PREC, int TERM, bool FILTER = false>
+__device__ bool base_pipelined(const SearchParams& p, WarpSmem& s, uint32_t& phase, int lane, Counters& ct,
+                               PhaseClock& pc, uint32_t ep, float d0, int& psize, HeapState& hs,
+                               uint32_t& status, uint32_t qi, float qn, bool ep_ok = true) {
+    const uint32_t skip_id = FILTER && !ep_ok ? ep : INVALID_ID;
+    TermState ts;
+    // the entry point is pushed and popped at once (hnswalg.h:325-359)
+    hs.live = EXACT && !p.lazy_heaps;
+    if (lane == 0 && (!FILTER || ep_ok)) {
+        s.pool[0] = mkkey(d0, ep) | (hs.live ? 0u : EXP_BIT);
+        if (EXACT) s.topheap[0] = mkkey(d0, ep);
+    }
+    psize = !FILTER || ep_ok ? 1 : 0;
+    __syncwarp();
+    const Counters before = ct;
+    Beam b;
+    auto enter = [&]() {
+        const LinkRow row = load_links(p, ep, lane);
+        fetch_rows<PREC, FILTER>(p, s, row.a, lane, b.f, skip_id);
+        b.rest = row.b;
+        b.guess = LinkRow{INVALID_ID, INVALID_ID};
+        b.guess_id = INVALID_ID;
+        b.hint_p = 0;
+        ct.l0_exp += 1;
+    };
+    int r = kBeamTie;
+    if (!EXACT || !hs.live) {
+        enter();
+        PT_MARK(3);
+        r = beam_loop<SPACE, FAST16, EXACT, PREC, TERM, FILTER, false>(p, s, phase, lane, ct, pc, b, d0, psize, hs, status,
+                                                                       qi, qn, skip_id, ts);
+        const int k = (int)p.k;
+        if (EXACT && r == kBeamDone && psize > k && khi(s.pool[k - 1]) == khi(s.pool[k])) r = kBeamTie;  // (c)
+        if (EXACT && r == kBeamTie) {
+            // start over with the heaps
+            ct = before;
+            __syncwarp();
+            for (uint32_t i = lane; i < 1u << p.log2_vis; i += 32) s.vis[i] = INVALID_ID;
+            __syncwarp();
+            if (lane == 0) {
+                s.vis[vis_slot(ep, p.log2_vis)] = ep;
+                s.pool[0] = mkkey(d0, ep);
+            }
+            __syncwarp();
+            hs.live = true;
+            psize = 1;
+        }
+    }
+    if (EXACT && r == kBeamTie) {
+        enter();
+        r = beam_loop<SPACE, FAST16, EXACT, PREC, TERM, FILTER, EXACT>(p, s, phase, lane, ct, pc, b, d0, psize, hs, status,
+                                                                       qi, qn, skip_id, ts);
+    }
+    if (r == kBeamFailed) return false;
     if (TERM == 1) term_final_row<SPACE>(p, s, lane, qi, ct.l0_exp, ct.l0_dists, psize, d0, qn, ts);
     return true;
 }
@@ -983,10 +1134,10 @@ __device__ bool base_pipelined(const SearchParams& p, WarpSmem& s, uint32_t& pha
 // reference's summation order; the pool is then re-sorted by the exact
 // (distance, id) keys, so the k returned distances are bit-exact.
 template <int SPACE>
-__device__ bool rerank_fp32(const SearchParams& p, WarpSmem& s, uint32_t& phase, int lane, const float4* qr,
-                            int& psize) {
+__device__ bool rerank_fp32(const SearchParams& p, WarpSmem& s, uint32_t& phase, int lane, int& psize) {
     const int R = min(psize, (int)p.rerank);
-    const RowSrc rs{reinterpret_cast<const unsigned char*>(p.vecs), p.row_bytes, p.stage_stride * 4, p.rr_slots};
+    const RowSrc rs{reinterpret_cast<const unsigned char*>(p.vecs), p.row_bytes, p.stage_stride * 4, p.rr_slots,
+                    p.gather ? &p.vmap : nullptr};
 #ifdef HNSWGPU_BOUNDS_CHECK
     for (int r = lane; r < psize; r += 32)
         for (int t = 0; t < psize; t++)
@@ -997,9 +1148,10 @@ __device__ bool rerank_fp32(const SearchParams& p, WarpSmem& s, uint32_t& phase,
         const int nb = min((int)rs.slots, R - b);
         uint32_t id = lane < nb ? kid(s.pool[b + lane]) : 0u;
         if (!DBG_OK(id < p.count && b + lane < (int)p.pool_cap, 70, id, b + lane)) id = 0;
-        if (!stage_src(p, s, phase, rs, lane < nb, id, lane, nb, lane)) return false;
+        copy_rows(p, s, rs, id, 0, nb, lane);
+        if (!copies_done(s, phase)) return false;
         float dc = 0.f;
-        batch_dist<SPACE>(p, s, qr, nb, 0, lane, dc);
+        batch_dist<SPACE, true>(p, s, nb, 0, lane, dc);
         __syncwarp();
         if (lane < nb) s.pool[b + lane] = mkkey(dc, id);
         __syncwarp();
@@ -1027,7 +1179,15 @@ __device__ bool rerank_fp32(const SearchParams& p, WarpSmem& s, uint32_t& phase,
     return true;
 }
 
-template <int SPACE, bool FAST16, bool EXACT, int PREC, int TERM, bool TIES = false, bool FILTER = false>
+// Whether the pipelined beam runs these parameters.  The general loop keeps
+// lists longer than 64 links, the reference order with deletions or a filter,
+// the epsilon search, and the learned stop outside dim % 16 == 0 and 32 links
+// (its checkpoints there see the beam before the next candidate is marked).
+__host__ __device__ __forceinline__ bool pipelined(const SearchParams& p, bool filter, bool fast16, int term) {
+    return (p.bare || filter) && !p.eps_mode && (term ? fast16 && p.maxM0 <= 32 : p.maxM0 <= 64);
+}
+
+template <int SPACE, bool FAST16, bool EXACT, int PREC, int TERM, bool FILTER = false>
 __device__ bool search_one(const SearchParams& p, WarpSmem& s, uint32_t& phase, uint32_t qi, int lane,
                            Counters& ct, PhaseClock& pc) {
     pc.start();
@@ -1094,13 +1254,13 @@ __device__ bool search_one(const SearchParams& p, WarpSmem& s, uint32_t& phase, 
     // (hnswalg.h:336-337) and never evaluated, so the exact-key lookup cannot
     // recognise it when the visited cache misses on it later: skip it by id.
     uint32_t skip_id = INVALID_ID;
-    // ef, or ef + 32 in tie-exact mode (ef + 1 in a tie-listing pass, for
-    // the pipelined beam only)
-    const int pcap = TIES ? (int)ef : (int)p.pool_cap;
+    const int pcap = (int)p.pool_cap;   // ef, or ef + 32 in tie-exact mode
     int tsz = 0, csz = 0;               // tie-exact mode: heap sizes (warp-uniform)
+    HeapState hs;
+    hs.live = EXACT;
     const uint64_t sentinel = mkkey(__int_as_float(0x7f7fffff), cur);
     // FILTER kernels run the id order only (the host never pairs it with EXACT)
-    const bool pipe = FAST16 && (bare || FILTER) && p.maxM0 <= 32 && !p.eps_mode;
+    const bool pipe = pipelined(p, FILTER, FAST16, TERM);
     float qn = 0.f;
     if (TERM) {  // |q|^2, a feature of the termination network
         for (uint32_t i = lane; i < p.dim; i += 32) qn = fmaf(s.q[i], s.q[i], qn);
@@ -1117,27 +1277,21 @@ __device__ bool search_one(const SearchParams& p, WarpSmem& s, uint32_t& phase, 
             // (approximate) arithmetic: a node re-reached after a visited-cache
             // miss is recognised by its exact (distance, id) key
             const RowSrc rs = trav_src<PREC>(p);
-            if (!stage_src(p, s, phase, rs, lane == 0, cur, 0, 1, lane)) return false;
+            copy_rows(p, s, rs, cur, 0, 1, lane);
+            if (!copies_done(s, phase)) return false;
             d0 = 0.f;
             batch_dist_lowp<SPACE, PREC>(p, s, 1, 0, lane, d0);
         }
         d0 = __shfl_sync(FULL, d0, 0);
         ct.l0_dists += 1;
         if (lane == 0) s.vis[vis_slot(cur, p.log2_vis)] = cur;
-        float4 qr[8];
-        const int n16 = (int)(p.dim >> 4);
-        const float4* q4 = reinterpret_cast<const float4*>(s.q);
-#pragma unroll
-        for (int c = 0; c < 8; c++) qr[c] = c < n16 ? q4[4 * c + (lane & 3)] : make_float4(0.f, 0.f, 0.f, 0.f);
         __syncwarp();
-        if (!base_pipelined<SPACE, EXACT, PREC, TERM, TIES, FILTER>(p, s, phase, lane, ct, pc, qr, cur, d0, psize,
-                                                                    tsz, status, qi, qn, bare || is_allowed(p, cur)))
+        if (!base_pipelined<SPACE, FAST16, EXACT, PREC, TERM, FILTER>(p, s, phase, lane, ct, pc, cur, d0, psize, hs,
+                                                                      status, qi, qn, bare || is_allowed(p, cur)))
             return false;
-        // (c): the reference pops top_candidates down to k by distance
-        if (TIES && psize > (int)p.k && khi(s.pool[p.k - 1]) == khi(s.pool[p.k])) status |= kTieBit;
-        if (PREC != 0 && !rerank_fp32<SPACE>(p, s, phase, lane, qr, psize)) return false;
+        tsz = hs.tsz;
+        if (PREC != 0 && !rerank_fp32<SPACE>(p, s, phase, lane, psize)) return false;
     } else {
-    if (TIES) status |= kTieBit;  // only the pipelined beam checks its ties
     if (bare || is_allowed(p, cur)) {
         float d0;
         if (!lane_distances<SPACE, FAST16>(p, s, phase, cur, 1, lane, d0, pc)) return false;
@@ -1317,7 +1471,7 @@ __device__ bool search_one(const SearchParams& p, WarpSmem& s, uint32_t& phase, 
                 int m = merge_sorted(s.pool, psize, pcap, pmask, key, posP, lane);
                 hint_p = min(hint_p, m);
             }
-            if (EXACT && nev) remove_keys(s.pool, psize, s.evbuf, nev, lane);
+            if (EXACT && nev) psize = remove_keys(s.pool, psize, s.evbuf, nev, lane);
             if (xmask) {
                 if (xsize + __popc(xmask) > xcap) status |= HNSWGPU_STATUS_OVERFLOW_BIT;
                 int m = merge_sorted(s.extra, xsize, xcap, xmask, key, posX, lane);
@@ -1365,7 +1519,7 @@ __device__ bool search_one(const SearchParams& p, WarpSmem& s, uint32_t& phase, 
         }
         return true;
     }
-    if (EXACT) {
+    if (EXACT && hs.live) {
         // the reference pops top_candidates down to k (hnswalg.h:1314-1316);
         // keep in the pool exactly the entries left in the heap
         int tn = tsz;
@@ -1396,7 +1550,7 @@ __device__ bool search_one(const SearchParams& p, WarpSmem& s, uint32_t& phase, 
     uint64_t* olab = p.out_labels + (size_t)qi * k;
     float* odist = p.out_dists + (size_t)qi * k;
     for (int r = lane; r < kk; r += 32) {
-        uint64_t e = s.pool[r];
+        uint64_t e = s.pool[r];  // (khi / kid ignore the expanded mark)
         if (!DBG_OK(kid(e) < p.count, 80 + (PREC << 2), kid(e), r)) e = 0;
         uint32_t dk = khi(e);
         uint64_t lab = p.labels[kid(e)];
@@ -1417,8 +1571,6 @@ __device__ bool search_one(const SearchParams& p, WarpSmem& s, uint32_t& phase, 
         olab[r] = ~0ull;
         odist[r] = __int_as_float(0x7f800000);
     }
-    if (TIES && (status & kTieBit) && lane == 0) p.tie_list[atomicAdd(p.tie_count, 1u)] = qi;
-    status &= ~kTieBit;
     if (lane == 0) {
         p.out_counts[qi] = kk;
         if (status) atomicOr(p.status, status);
@@ -1427,9 +1579,9 @@ __device__ bool search_one(const SearchParams& p, WarpSmem& s, uint32_t& phase, 
     return true;
 }
 
-template <int SPACE, bool FAST16, bool EXACT, int PREC, int TERM, bool TIES, bool FILTER>
+template <int SPACE, bool FAST16, bool EXACT, int PREC, int TERM, bool FILTER>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, PREC ? HNSWGPU_MINB_LOWP : kMinBlocks)
-    hnsw_search_kernel(SearchParams p) {
+    hnsw_search_kernel(const __grid_constant__ SearchParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char* base = smem + (size_t)warp * p.warp_smem;
@@ -1456,19 +1608,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, PREC ? HNSWGPU_MINB_LOWP 
     __syncwarp();
     uint32_t phase = 0;
     PhaseClock pc;
-    // a list pass runs the queries a previous launch on this stream listed
-    const uint32_t nrun = p.qcount ? min(*p.qcount, p.nq) : p.nq;
     while (true) {
         uint32_t qi = 0;
-        if (lane == 0) {
-            qi = atomicAdd(p.work_counter, 1u);
-            if (p.qlist && qi < nrun) qi = p.qlist[qi];
-            else if (qi >= nrun) qi = 0xffffffffu;
-        }
+        if (lane == 0) qi = atomicAdd(p.work_counter, 1u);
         qi = __shfl_sync(FULL, qi, 0);
         if (qi >= p.nq) break;
         Counters ct = {0, 0, 0, 0};
-        if (!search_one<SPACE, FAST16, EXACT, PREC, TERM, TIES, FILTER>(p, s, phase, qi, lane, ct, pc)) {
+        if (!search_one<SPACE, FAST16, EXACT, PREC, TERM, FILTER>(p, s, phase, qi, lane, ct, pc)) {
             if (lane == 0) atomicOr(p.status, HNSWGPU_STATUS_TIMEOUT_BIT);
             // wait (bounded) for this warp's copies still in flight, then leave
             mbar_wait(s.bar, phase);
@@ -1501,6 +1647,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, PREC ? HNSWGPU_MINB_LOWP 
 
 }  // namespace
 
+bool hnsw_pipelined(const SearchParams& p) { return pipelined(p, false, p.fast16 != 0, (int)p.term_mode); }
+
 size_t warp_smem_layout(SearchParams& p) {
     if (p.lean) return lean_smem_layout(p);
     size_t off = 16 + 128;  // mbarrier (8 bytes) + pad, then the 32-entry id compaction buffer
@@ -1508,7 +1656,9 @@ size_t warp_smem_layout(SearchParams& p) {
     off += (size_t)p.row_floats * 4;
     off = (off + 15) & ~(size_t)15;
     // staging area followed by the visited cache: after the beam the two
-    // together stage the float32 rows of the re-rank
+    // together stage the float32 rows of the re-rank (a gather's destination
+    // is 128-byte aligned and takes whole groups of four rows)
+    off = (off + 127) & ~(size_t)127;
     p.off_stage = (uint32_t)off;
     size_t stage = (size_t)p.stage_slots * p.stage_stride * 4;
     if (p.prec) stage = std::max(stage, (size_t)p.tslots * p.tstage_bytes);
@@ -1516,6 +1666,7 @@ size_t warp_smem_layout(SearchParams& p) {
     p.off_vis = (uint32_t)off;
     off += ((size_t)1 << p.log2_vis) * 4;
     p.rr_slots = p.prec ? (uint32_t)std::min<size_t>(32, (off - p.off_stage) / ((size_t)p.stage_stride * 4)) : 0;
+    if (p.gather) p.rr_slots &= ~3u;
     off = (off + 7) & ~(size_t)7;
     p.off_pool = (uint32_t)off;
     off += (size_t)p.pool_cap * 8;
@@ -1523,8 +1674,9 @@ size_t warp_smem_layout(SearchParams& p) {
     off += p.exact ? ((size_t)p.ef + 1) * 8 : 0;
     p.off_cand = (uint32_t)off;
     off += p.exact ? (size_t)p.cand_cap * 8 : 0;
+    off = (off + 15) & ~(size_t)15;
     p.off_acc = (uint32_t)off;
-    off += p.exact ? 32 * 8 : 0;
+    off += 32 * 8;
     p.off_ev = (uint32_t)off;
     off += p.exact ? 32 * 8 : 0;
     p.off_extra = (uint32_t)off;
@@ -1535,11 +1687,11 @@ size_t warp_smem_layout(SearchParams& p) {
 }
 
 namespace {
-template <int SPACE, bool FAST16, bool EXACT, int PREC, int TERM = 0, bool TIES = false, bool FILTER = false>
+template <int SPACE, bool FAST16, bool EXACT, int PREC, int TERM = 0, bool FILTER = false>
 cudaError_t launch_t(const SearchParams& p, int num_sms, cudaStream_t stream, int* blocks_out) {
     // per-instantiation, per-device cache of the opt-in shared-memory size and occupancy
     static LaunchCache cache;
-    const void* fn = (const void*)hnsw_search_kernel<SPACE, FAST16, EXACT, PREC, TERM, TIES, FILTER>;
+    const void* fn = (const void*)hnsw_search_kernel<SPACE, FAST16, EXACT, PREC, TERM, FILTER>;
     const size_t smem = (size_t)p.warp_smem * kWarpsPerBlock;
     int occ_per_sm = 0;
     cudaError_t e = cache.blocks_per_sm(fn, kWarpsPerBlock * 32, smem, &occ_per_sm);
@@ -1550,7 +1702,7 @@ cudaError_t launch_t(const SearchParams& p, int num_sms, cudaStream_t stream, in
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
     if (blocks_out) *blocks_out = (int)blocks;
-    hnsw_search_kernel<SPACE, FAST16, EXACT, PREC, TERM, TIES, FILTER>
+    hnsw_search_kernel<SPACE, FAST16, EXACT, PREC, TERM, FILTER>
         <<<(unsigned)blocks, kWarpsPerBlock * 32, smem, stream>>>(p);
     return cudaGetLastError();
 }
@@ -1642,13 +1794,15 @@ cudaError_t launch_wait_timeout_selftest(uint32_t limit, uint32_t* status, cudaS
     return cudaGetLastError();
 }
 
-// Pipelined beam over an index with deletions and / or a filter (id order,
-// dim % 16 == 0, maxM0 <= 32; learned stop or none).
+// Pipelined beam over an index with deletions and / or a filter (id order;
+// learned stop or none).
 template <int SPACE, int TERM>
 cudaError_t launch_filter_t(const SearchParams& p, int num_sms, cudaStream_t stream, int* blocks_out) {
-    if (p.prec == 0) return launch_t<SPACE, true, false, 0, TERM, false, true>(p, num_sms, stream, blocks_out);
-    return p.prec == 1 ? launch_t<SPACE, true, false, 1, TERM, false, true>(p, num_sms, stream, blocks_out)
-                       : launch_t<SPACE, true, false, 2, TERM, false, true>(p, num_sms, stream, blocks_out);
+    if (p.prec == 0)
+        return p.fast16 ? launch_t<SPACE, true, false, 0, TERM, true>(p, num_sms, stream, blocks_out)
+                        : launch_t<SPACE, false, false, 0, TERM, true>(p, num_sms, stream, blocks_out);
+    return p.prec == 1 ? launch_t<SPACE, true, false, 1, TERM, true>(p, num_sms, stream, blocks_out)
+                       : launch_t<SPACE, true, false, 2, TERM, true>(p, num_sms, stream, blocks_out);
 }
 template <int SPACE>
 cudaError_t launch_filter(const SearchParams& p, int num_sms, cudaStream_t stream, int* blocks_out) {
@@ -1658,18 +1812,9 @@ cudaError_t launch_filter(const SearchParams& p, int num_sms, cudaStream_t strea
 
 cudaError_t launch_hnsw_search(const SearchParams& p, int space, int num_sms, cudaStream_t stream, int* blocks_out) {
     if (p.lean) return lean_eligible(p) ? launch_hnsw_lean(p, space, num_sms, stream, blocks_out) : cudaErrorInvalidValue;
-    if (!p.bare && !p.exact && p.fast16 && p.maxM0 <= 32 && p.term_mode != 1 && !p.tie_list)
+    if (!p.bare && !p.exact && p.term_mode != 1 && pipelined(p, true, p.fast16 != 0, (int)p.term_mode))
         return space == 0 ? launch_filter<0>(p, num_sms, stream, blocks_out)
                           : launch_filter<1>(p, num_sms, stream, blocks_out);
-    if (p.tie_list) {
-        // id-order beam that lists its tie-steered queries (float32, 4-lane
-        // distances, no filter or deletes: checked by the host)
-        if (p.exact || p.prec || p.term_mode || !p.fast16 || !p.bare || p.maxM0 > 32 || p.pool_cap != p.ef + 1 ||
-            !p.tie_count)
-            return cudaErrorInvalidValue;
-        return space == 0 ? launch_t<0, true, false, 0, 0, true>(p, num_sms, stream, blocks_out)
-                          : launch_t<1, true, false, 0, 0, true>(p, num_sms, stream, blocks_out);
-    }
     if (p.term_mode) return space == 0 ? launch_term<0>(p, num_sms, stream, blocks_out)
                                        : launch_term<1>(p, num_sms, stream, blocks_out);
     if (p.prec) return space == 0 ? launch_lowp<0>(p, num_sms, stream, blocks_out)

@@ -1,5 +1,6 @@
 // Launch parameters of the HNSW search kernel (shared by host and device).
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstddef>
@@ -68,9 +69,11 @@ cudaError_t term_logits(const float* params, const float* feats, uint64_t n, flo
 constexpr int kMinBlocks = HNSWGPU_MINB;     // launch bound: resident CTAs per SM
 constexpr uint32_t HNSWGPU_STATUS_TIMEOUT_BIT = 0x1u;
 constexpr uint32_t HNSWGPU_STATUS_OVERFLOW_BIT = 0x2u;
-constexpr uint32_t kTieBit = 0x80000000u;  // per-query, never reported: the run met a steering tie
 
 struct SearchParams {
+    // rows as tensor maps for gathers of four (gather / tgather: whether they fit one)
+    alignas(64) CUtensorMap vmap, tmap;
+    uint32_t gather, tgather;
     // index (device pointers)
     const float* vecs;            // count x row_floats, rows zero-padded
     const uint32_t* links0;       // count x maxM0 ids, unused slots = 0xffffffff
@@ -95,7 +98,7 @@ struct SearchParams {
     uint32_t eps_mode;            // 1: stop once a candidate lies beyond eps with eps_min items held
     float eps;                    // epsilon (a distance, squared for L2)
     uint32_t eps_min;             // min_num_candidates
-    uint32_t pool_cap;            // ef (canonical) or ef + 32 (tie-exact)
+    uint32_t pool_cap;            // ef (id order) or ef + 32 (tie-exact)
     uint32_t cand_cap;            // tie-exact: candidate heap entries in shared memory
     uint32_t cand_spill_cap;      // tie-exact: further entries per warp in cand_spill
     uint32_t cand_spill_warps;    // warps that cand_spill has room for
@@ -108,13 +111,7 @@ struct SearchParams {
     uint32_t* work_counter;       // zero at launch; reset to zero by the last block
     uint32_t* done_counter;       // blocks finished (same slot discipline)
     uint32_t* status;
-    // tie-exact mode in two passes: the id-order beam lists the queries whose
-    // run met a distance tie that can steer the reference's heaps, then the
-    // heap replay runs on those queries only
-    uint32_t* tie_list;           // first pass: flagged query indices (null: no listing)
-    uint32_t* tie_count;          // first pass: entries appended to tie_list (zero at launch)
-    const uint32_t* qlist;        // second pass: query indices to run (null: 0 .. nq - 1)
-    const uint32_t* qcount;       // second pass: device word holding the entries of qlist
+    uint32_t lazy_heaps;          // tie-exact pipelined beam: heaps only for queries with a tie that can matter
     unsigned long long* phase_cycles;  // 10 counters, profiling builds only (may be null)
     // learned early termination (mode 1 = record checkpoints, 2 = stop early)
     uint32_t term_mode;
@@ -156,6 +153,8 @@ cudaError_t noalloc_scratch_address(int device, uint32_t** out);
 // *status (device memory).
 cudaError_t launch_wait_timeout_selftest(uint32_t limit, uint32_t* status, cudaStream_t stream);
 
+// Whether an unfiltered search runs in the pipelined beam.
+bool hnsw_pipelined(const SearchParams& p);
 // Fills the off_* fields and warp_smem from the sizes; returns warp_smem.
 size_t warp_smem_layout(SearchParams& p);
 // The lean fp8 beam's per-warp layout (called by warp_smem_layout when p.lean).

@@ -447,14 +447,24 @@ hnswgpu::SearchParams hnsw_params(const hnswgpu_index* h, const float* dq, uint6
     p.out_dists = dd;
     p.out_counts = dc;
     p.trace = dtrace;
-    // Staging rows: the 4-lanes-per-row path reads 8 rows per LDS.128 pass, a
-    // row pad of 16 floats puts consecutive rows half a bank cycle apart
-    // (conflict-free quarter warps); the one-lane-per-row path wants 4.
+    // Staging rows: 4 lanes read one row, 8 rows a pass.  Where they read 16
+    // bytes each (16 accumulators), a stride of 16 floats modulo 32 puts the two
+    // rows of a quarter warp on disjoint banks; where they read 4 bytes each (4
+    // or 8 accumulators), 8 modulo 32 leaves two rows to a bank (4 would spread
+    // all 8, but a group of four gathered rows starts on 128 bytes).
     p.fast16 = (h->dim % 16 == 0) ? 1u : 0u;
     p.links_unique = h->links_unique ? 1u : 0u;
-    p.stage_stride = h->row_floats + (p.fast16 ? 16u : 4u);
+    {
+        const bool by16 = p.fast16 || (h->dim > 16 && h->dim % 4 != 0);
+        p.stage_stride = h->row_floats + (((by16 ? 16u : 8u) - h->row_floats) & 31u);
+    }
+    p.gather = p.stage_stride <= 256 ? 1u : 0u;
     uint32_t slots = (uint32_t)((9u * 1024u + 512u) / (p.stage_stride * 4));
-    p.stage_slots = std::max(1u, std::min(p.fast16 ? (uint32_t)HNSWGPU_FP32_SLOTS : 32u, slots));
+    p.stage_slots = std::max(1u, std::min((uint32_t)HNSWGPU_FP32_SLOTS, slots));
+    if (p.gather) {  // whole groups of four
+        p.stage_slots = std::max(4u, p.stage_slots & ~3u);
+        cuda_check(hnswgpu::gather_map(h->vecs.p, h->count, p.row_bytes, p.stage_stride * 4, &p.vmap), "tensor map (rows)");
+    }
     p.extra_cap = p.bare ? 0u : std::max<uint32_t>(128u, 4u * p.ef);
     p.exact = exact ? 1u : 0u;
     p.pool_cap = exact ? p.ef + 32u : p.ef;
@@ -486,6 +496,10 @@ hnswgpu::SearchParams hnsw_params(const hnswgpu_index* h, const float* dq, uint6
         if ((st & 1) == 0) st++;
         p.tstage_bytes = st * 64;
         p.tslots = prec == 2 ? 32u : 16u;
+        p.tgather = p.tstage_bytes <= 1024 ? 1u : 0u;
+        if (p.tgather)
+            cuda_check(hnswgpu::gather_map(h->tcopy[prec].p, h->count, p.trow_bytes, p.tstage_bytes, &p.tmap),
+                       "tensor map (traversal rows)");
         p.stage_slots = 8;  // float32 rows: upper-layer descent and re-rank batches
         p.rerank = (uint32_t)std::max<uint64_t>(k, rerank ? std::min<uint64_t>(rerank, p.ef) : p.ef);
 #ifdef HNSWGPU_BOUNDS_CHECK
@@ -502,7 +516,7 @@ hnswgpu::SearchParams hnsw_params(const hnswgpu_index* h, const float* dq, uint6
     size_t ws = hnswgpu::warp_smem_layout(p);
     int max_optin = 0;
     cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attr");
-    while (!p.lean && ws * wpb > (size_t)max_optin && p.log2_vis > 8) {
+    while (!p.lean && ws * wpb > (size_t)max_optin && p.log2_vis > 7) {
         p.log2_vis--;
         ws = hnswgpu::warp_smem_layout(p);
     }
@@ -578,79 +592,50 @@ static void take_counter_slot(hnswgpu_index* h, hnswgpu::SearchParams& p) {
     p.done_counter = h->counters.p + 2 * slot + 1;
 }
 
-// Two-pass tie-exact mode: the replay pass runs one query per warp and takes
-// about one replayed query's latency, whatever the share listed.  Above this
-// share of listed queries (e.g. integer-valued data at large ef) the single
-// pass that replays every query is the faster one.
-constexpr float kTwoPassMaxShare = 0.3f;
-
-// Fold in the listed share of the last listing pass once its copy landed.
-static void poll_tie_share(hnswgpu_index* h) {
-    if (!h->tie_pending_nq) return;
-    const cudaError_t e = cudaEventQuery(h->tie_ev);
-    if (e == cudaErrorNotReady) {
-        if (cudaPeekAtLastError() == cudaErrorNotReady) (void)cudaGetLastError();
-        return;
-    }
-    cuda_check(e, "cudaEventQuery");
-    h->tie_share[h->tie_pending_ef] = {(float)*h->tie_host / (float)h->tie_pending_nq, 0u};
-    h->tie_pending_nq = 0;
+// A batch that leaves shared memory unused takes larger staging batches (up
+// to one whole list): the rows of an expansion then come in one wait.  A row of
+// 768 floats has room for 3 of them in the 9.5 KB that 15 resident warps leave
+// each other, so 100 such queries waited 7 times an expansion.
+static void widen_staging(hnswgpu_index* h, hnswgpu::SearchParams& p, uint64_t nq) {
+    if (p.prec || p.lean) return;
+    int sm_smem = 0, reserved = 0, max_optin = 0;
+    cuda_check(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device), "attr");
+    cuda_check(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, h->device), "attr");
+    cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attr");
+    const uint64_t per_sm = (nq + (uint64_t)h->num_sms - 1) / (uint64_t)h->num_sms;
+    const uint64_t room = std::min<uint64_t>((uint64_t)sm_smem / per_sm, (uint64_t)(max_optin + reserved));
+    if (room <= (uint64_t)p.warp_smem + (uint64_t)reserved) return;
+    const uint64_t more = (room - p.warp_smem - (uint64_t)reserved) / ((uint64_t)p.stage_stride * 4);
+    const uint32_t list = (uint32_t)std::min<uint64_t>(32, (p.maxM0 + 3) / 4 * 4);
+    const uint32_t slots = std::min<uint32_t>(list, (uint32_t)std::min<uint64_t>(64, p.stage_slots + more)) & ~3u;
+    if (slots <= p.stage_slots) return;
+    p.stage_slots = slots;
+    hnswgpu::warp_smem_layout(p);
 }
 
-// One HNSW search on device buffers, scratch from the index.  The tie-exact
-// mode of an unfiltered float32 beam runs in two launches: the id-order beam
-// answers every query and lists those whose run met a tie that can steer the
-// reference's heaps (for the others the two orders make the same decisions, so
-// the results are the reference's); the heap replay then reruns only the
-// listed queries, reading the list's length on the device.
+// One HNSW search on device buffers, scratch from the index.  wide: the caller
+// waits for the result, so no other batch of this index shares the SMs.
 void run_hnsw(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint64_t ef, const uint8_t* dallow,
               uint64_t* dl, float* dd, int32_t* dc, uint32_t* dtrace, cudaStream_t st, bool exact, uint32_t prec,
-              uint32_t rerank, const TermCfg* term, bool replay_all) {
+              uint32_t rerank, const TermCfg* term, bool replay_all, bool wide) {
     if (prec) ensure_traversal_copy(h, prec);
     hnswgpu::SearchParams p = hnsw_params(h, dq, nq, k, ef, dallow, dl, dd, dc, dtrace, exact, prec, rerank, true);
     apply_term(h, p, term);
     p.status = h->status.p;
     const int space = kspace(h);
-    hnswgpu::SearchParams p1{};
-    bool two_pass = exact && !replay_all && p.fast16 && p.bare && p.maxM0 <= 32;
-    if (two_pass) {
-        // a share measured above the bound picks the single pass; every 64th
-        // call at that ef measures it again
-        poll_tie_share(h);
-        auto it = h->tie_share.find(p.ef);
-        if (it != h->tie_share.end() && it->second.share > kTwoPassMaxShare && ++it->second.calls % 64 != 0)
-            two_pass = false;
-    }
-    if (two_pass) {
-        // the listing pass merges into ef + 1 slots to see the first entry dropped
-        p1 = hnsw_params(h, dq, nq, k, ef, dallow, dl, dd, dc, dtrace, false);
-        p1.pool_cap = p1.ef + 1;
-        int max_optin = 0;
-        cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attr");
-        two_pass = hnswgpu::warp_smem_layout(p1) * hnswgpu::kWarpsPerBlock <= (size_t)max_optin;
-    }
-    if (two_pass) {
-        p1.status = h->status.p;
-        if (h->tie_list.n < nq + 1) {
-            cuda_check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
-            h->tie_list.alloc(nq + 1);
-        }
-        cuda_check(cudaMemsetAsync(h->tie_list.p, 0, 4, st), "cudaMemsetAsync");
-        p1.tie_count = h->tie_list.p;
-        p1.tie_list = h->tie_list.p + 1;
-        take_counter_slot(h, p1);
-        cuda_check(hnswgpu::launch_hnsw_search(p1, space, h->num_sms, st, nullptr), "hnsw_search launch");
-        p.qcount = h->tie_list.p;
-        p.qlist = h->tie_list.p + 1;
-        if (!h->tie_pending_nq) {
-            if (!h->tie_host) cuda_check(cudaHostAlloc((void**)&h->tie_host, 4, cudaHostAllocDefault), "cudaHostAlloc");
-            if (!h->tie_ev) cuda_check(cudaEventCreateWithFlags(&h->tie_ev, cudaEventDisableTiming), "cudaEventCreate");
-            cuda_check(cudaMemcpyAsync(h->tie_host, h->tie_list.p, 4, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
-            cuda_check(cudaEventRecord(h->tie_ev, st), "cudaEventRecord");
-            h->tie_pending_ef = p.ef;
-            h->tie_pending_nq = nq;
+    if (exact && !replay_all && p.bare && hnswgpu::hnsw_pipelined(p)) {
+        p.lazy_heaps = 1u;
+        if (nq > 8ull * (uint64_t)h->num_sms) {
+            // few queries need their heaps: all but the top of the candidate
+            // heap goes to the spill area, for the sake of residency (a small
+            // batch waits for the slowest query, heaps and all)
+            const uint32_t cap = p.cand_cap + p.cand_spill_cap;
+            p.cand_cap = std::min(p.cand_cap, 32u);
+            p.cand_spill_cap = cap - p.cand_cap;
+            hnswgpu::warp_smem_layout(p);
         }
     }
+    if (wide) widen_staging(h, p, nq);
     if (exact) attach_spill(h, p, st);
 #ifdef HNSWGPU_PHASE_TIMING
     static unsigned long long* phase_buf = nullptr;
@@ -1101,7 +1086,7 @@ void run_search(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint
     } else if (h->is_bf || scan) {
         run_bf_exact(h, dq, nq, k, dallow, dl, dd, dc, st, may_sync);
     } else {
-        run_hnsw(h, dq, nq, k, ef, dallow, dl, dd, dc, dtrace, st, exact, prec, rerank, term, replay_all);
+        run_hnsw(h, dq, nq, k, ef, dallow, dl, dd, dc, dtrace, st, exact, prec, rerank, term, replay_all, may_sync);
     }
 }
 
@@ -1751,7 +1736,7 @@ int hnswgpu_search_checkpoints(hnswgpu_index* h, const float* queries, uint64_t 
         term.dists = out_ckpt_dists ? dx.p : nullptr;
         term.count = dn.p;
         run_hnsw(h, dq.p, nq, k, ef, nullptr, dl.p, dd.p, dc.p, nullptr, st, false, o.precision, o.rerank, &term,
-                 false);
+                 false, false);
         cuda_check(cudaMemcpyAsync(out_labels, dl.p, nq * k * 8, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
         cuda_check(cudaMemcpyAsync(out_dists, dd.p, nq * k * 4, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
         cuda_check(cudaMemcpyAsync(out_counts, dc.p, nq * 4, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");

@@ -89,17 +89,6 @@ struct hnswgpu_index {
     DevBuf<unsigned char> tcopy[3];  // low-precision traversal copies (index 1 bf16, 2 fp8)
     DevBuf<unsigned char> term_model;  // learned termination: packed network
     DevBuf<uint64_t> cand_spill;       // tie-exact mode: candidate-heap tails
-    DevBuf<uint32_t> tie_list;         // tie-exact mode: [0] count, then the queries to replay
-    // share of listed queries per ef, read back without blocking: the word
-    // tie_list[0] is copied to pinned memory after a listing pass
-    uint32_t* tie_host = nullptr;
-    cudaEvent_t tie_ev = nullptr;
-    uint64_t tie_pending_ef = 0, tie_pending_nq = 0;
-    struct TieShare {
-        float share = 0.f;
-        uint32_t calls = 0;  // one-pass calls since the share was measured
-    };
-    std::unordered_map<uint64_t, TieShare> tie_share;
     DevBuf<float2> tc_rowinfo[3];      // tensor-core brute force: (|x|^2, scale) per row and precision
     // tensor-core brute force: per-call workspace
     DevBuf<float> tc_qf, tc_qscale, tc_tau, tc_part;
@@ -119,8 +108,6 @@ struct hnswgpu_index {
     // search can hold it while it reads that state
     mutable std::mutex mu;
     ~hnswgpu_index() {
-        if (tie_host) cudaFreeHost(tie_host);
-        if (tie_ev) cudaEventDestroy(tie_ev);
         if (pool) cudaMemPoolDestroy(pool);
     }
     uint64_t device_bytes() const {

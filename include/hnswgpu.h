@@ -71,13 +71,14 @@ extern "C" {
                                      that exact distance ties resolve as in
                                      hnswlib (results identical to searchKnn);
                                      without it ties break by internal id.
-                                     Runs in two passes: the id-order beam for
-                                     every query, then the heap replay only for
-                                     the queries whose run met a distance tie
-                                     that can steer the reference's heaps.     */
-#define HNSWGPU_REPLAY_ALL 0x20u  /* with HNSWGPU_EXACT_TIES: one pass, the
-                                     heap replay for every query (same results;
-                                     for testing and measurement).             */
+                                     Every query first runs the id-order beam;
+                                     those whose run met a distance tie that can
+                                     change the result run again with the
+                                     reference's heaps.                        */
+#define HNSWGPU_REPLAY_ALL 0x20u  /* with HNSWGPU_EXACT_TIES: the heap replay
+                                     for every query, without the id-order beam
+                                     (same results; for testing and
+                                     measurement).                             */
 #define HNSWGPU_LEARNED_STOP 0x8u /* HNSW: end each query's level-0 beam when
                                      the termination network set by
                                      hnswgpu_set_termination_model judges its
@@ -294,7 +295,7 @@ HNSWGPU_API int hnswgpu_search_epsilon(hnswgpu_index* index, const float* querie
  * Same search as hnswgpu_search with HNSWGPU_DEVICE_PTRS: queries, outputs and
  * the optional allow mask are device pointers, `ef` 0 means the index's ef,
  * flags may only hold HNSWGPU_EXACT_TIES (which here always runs the one-pass
- * heap replay: the two-pass form needs a per-query list); the call is
+ * heap replay for every query); the call is
  * asynchronous on `stream`.  It holds the index's lock while it reads the
  * index, so it may run beside set_ef / mark_deleted in other threads.
  * The kernel's scratch (work counter, finished-CTA counter, status word) is a
