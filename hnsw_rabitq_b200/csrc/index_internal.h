@@ -55,6 +55,8 @@ struct DevBuf {
 
 }  // namespace hnswgpu_host
 
+constexpr size_t kPinBytes = 2u << 20;
+
 struct hnswgpu_index {
     template <class T>
     using DevBuf = hnswgpu_host::DevBuf<T>;
@@ -84,6 +86,7 @@ struct hnswgpu_index {
     uint32_t next_counter = 0;
     DevBuf<uint32_t> status;
     DevBuf<unsigned char> io;  // host-pointer calls: queries + outputs
+    unsigned char* pinned = nullptr;  // small host-pointer calls: kPinBytes, queries in the first half, outputs in the second
     DevBuf<uint8_t> allow;
     DevBuf<float> bf_norms;    // brute force: per-row helper values
     DevBuf<unsigned char> tcopy[3];  // low-precision traversal copies (index 1 bf16, 2 fp8)
@@ -108,6 +111,7 @@ struct hnswgpu_index {
     // search can hold it while it reads that state
     mutable std::mutex mu;
     ~hnswgpu_index() {
+        if (pinned) cudaFreeHost(pinned);
         if (pool) cudaMemPoolDestroy(pool);
     }
     uint64_t device_bytes() const {
