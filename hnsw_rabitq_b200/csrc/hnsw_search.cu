@@ -144,11 +144,6 @@ __device__ __forceinline__ bool copies_done(const WarpSmem& s, uint32_t& phase) 
     return __all_sync(FULL, ok);
 }
 
-__device__ __forceinline__ void prefetch_row(const RowSrc& r, uint32_t id) {
-    const unsigned char* x = r.base + (uint64_t)id * r.row_bytes;
-    for (uint32_t o = 0; o < r.row_bytes; o += 128) prefetch_l2(x + o);
-}
-
 __device__ __forceinline__ bool is_allowed(const SearchParams& p, uint32_t id) {
     if (p.deleted_bits && ((p.deleted_bits[id >> 5] >> (id & 31)) & 1u)) return false;
     if (p.allow && !p.allow[id]) return false;
@@ -452,7 +447,9 @@ __device__ __forceinline__ bool lane_distances(const SearchParams& p, const Warp
 // first TMA batch are issued before the pool merge / heap operations of the
 // current expansion, which then run under that memory latency.  The list of
 // the candidate after that is loaded a whole expansion ahead (it is the right
-// one unless a closer neighbour turns up), and its rows are pulled into L2.
+// one unless a closer neighbour turns up).  Pulling rows into L2 ahead of their
+// copies cost more instructions than it saved waiting: the rows of that list
+// 5-7 %, those of a later batch or of a list's second half 1-3 %.
 struct Fetch {
     uint32_t id;     // this lane's neighbour id (link order), or INVALID_ID
     bool fresh;      // evaluated now (missed in the visited cache)
@@ -505,15 +502,6 @@ __device__ __forceinline__ void fetch_rows(const SearchParams& p, WarpSmem& s, u
     f.cid2 = s.cbuf[lane];
     f.n0 = min((int)rs.slots, f.nnew);
     if (f.n0 > 0) copy_rows(p, s, rs, f.cid2, 0, f.n0, lane);
-    if (lane >= f.n0 && lane < f.nnew) prefetch_row(rs, f.cid2);  // rows of the later batches: into L2 meanwhile
-}
-
-// Start pulling the rows of a list that will probably be expanded soon into L2
-// (those the visited cache does not hold).
-template <int PREC>
-__device__ __forceinline__ void prefetch_rows(const SearchParams& p, const WarpSmem& s, uint32_t id) {
-    const RowSrc rs = trav_src<PREC>(p);
-    if (id != INVALID_ID && s.vis[vis_slot(id, p.log2_vis)] != id) prefetch_row(rs, id);
 }
 
 // Approximate distances from staged low-precision rows [0, n) into the
@@ -596,10 +584,10 @@ __device__ __forceinline__ void batch_dist_lowp(const SearchParams& p, const War
 }
 
 // Distances of all fresh neighbours of a fetched list; result in the owning
-// (link-order) lane.  `guess`: a link of the list most likely fetched next.
+// (link-order) lane.
 template <int SPACE, bool FAST16, int PREC>
 __device__ __forceinline__ bool fetch_distances(const SearchParams& p, const WarpSmem& s, uint32_t& phase,
-                                                const Fetch& f, int lane, float& d, uint32_t guess, PhaseClock& pc) {
+                                                const Fetch& f, int lane, float& d, PhaseClock& pc) {
     float dc = __int_as_float(0x7f800000);
     const RowSrc rs = trav_src<PREC>(p);
     for (int s0 = 0; s0 < f.nnew; s0 += (int)rs.slots) {
@@ -607,7 +595,6 @@ __device__ __forceinline__ bool fetch_distances(const SearchParams& p, const War
         if (s0) copy_rows(p, s, rs, f.cid2, s0, n, lane);
         if (!copies_done(s, phase)) return false;
         PT_MARK(4);
-        if (s0 == 0) prefetch_rows<PREC>(p, s, guess);  // (its list has arrived with the rows)
         if (PREC == 0) batch_dist<SPACE, FAST16>(p, s, n, s0, lane, dc);
         else batch_dist_lowp<SPACE, PREC>(p, s, n, s0, lane, dc);
         PT_MARK(5);
@@ -832,7 +819,7 @@ __device__ __forceinline__ int beam_loop(const SearchParams& p, WarpSmem& s, uin
     while (true) {
         float d;
         ct.l0_dists += b.f.nnew;
-        if (!fetch_distances<SPACE, FAST16, PREC>(p, s, phase, b.f, lane, d, LIVE ? INVALID_ID : b.guess.a, pc))
+        if (!fetch_distances<SPACE, FAST16, PREC>(p, s, phase, b.f, lane, d, pc))
             return kBeamFailed;
         const Fetch& f = b.f;
         // ---- acceptance (closed form of hnswalg.h:395 over the link order)
@@ -941,7 +928,6 @@ __device__ __forceinline__ int beam_loop(const SearchParams& p, WarpSmem& s, uin
                 if (!inner) row = !LIVE && next == b.guess_id ? b.guess : load_links(p, next, lane);
                 b.rest = row.b;
                 fetch_rows<PREC, FILTER>(p, s, row.a, lane, fn, skip_id);
-                prefetch_rows<PREC>(p, s, row.b);  // (none but in a list of more than 32 links)
             }
         }
         PT_MARK(2);
