@@ -405,8 +405,18 @@ __device__ __forceinline__ void batch_dist(const SearchParams& p, const WarpSmem
         const float4* x4 = reinterpret_cast<const float4*>(row_of(g + (lane >> 2))) + a;
         const float4* y4 = reinterpret_cast<const float4*>(row_of(g + 8 + (lane >> 2))) + a;
         float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+        int c = 0;
+        // long rows: more reads in flight (not worth the code for short ones)
+#pragma unroll 1
+        for (; n16 > 8 && c + 4 <= n16; c += 4)
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float4 qv = q4[4 * (c + u)];
+                acc_chunk<SPACE>(qv, x4[4 * (c + u)], c0);
+                acc_chunk<SPACE>(qv, y4[4 * (c + u)], c1);
+            }
 #pragma unroll 2
-        for (int c = 0; c < n16; c++) {
+        for (; c < n16; c++) {
             const float4 qv = q4[4 * c];
             acc_chunk<SPACE>(qv, x4[4 * c], c0);
             acc_chunk<SPACE>(qv, y4[4 * c], c1);
