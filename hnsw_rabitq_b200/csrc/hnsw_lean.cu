@@ -46,18 +46,18 @@
 #include "launch_cache.h"
 #include "term_mlp.cuh"
 
-// launch bound, resident 2-warp CTAs per SM.  On the 1M x 128 workload a
-// bound of 10 (96 registers, 20 query warps) was 9 % faster than 8 (128
-// registers); 11 and 12 were slower.  With a bound of 9 the compiler still
-// allocates 96 registers (10 CTAs reside) but schedules the loop differently,
-// 2 % faster than the bound of 10 (same-box A/B)
+// launch bound, resident 1-warp CTAs per SM (96 registers, 20 query warps
+// reside).  One warp per CTA instead of two: a CTA gives its shared memory back
+// when its own query is done (500k x 128, ef 52, a call: 100 queries 233 -> 224
+// us, 10k 1.30 -> 1.28 ms).  Bounds of 16 and 20 were 7 % and 3 % slower than
+// 18: the compiler schedules the loop differently for each.
 #ifndef HNSWGPU_MINB_LEAN
-#define HNSWGPU_MINB_LEAN 9
+#define HNSWGPU_MINB_LEAN 18
 #endif
 
 // Where the learned-stop kernels read the packed network: 1 = one copy in
 // shared memory per 4-warp CTA (residency 16 warps per SM), 0 = through the
-// read-only cache from 2-warp CTAs (the fixed-ef residency).
+// read-only cache from 1-warp CTAs (the fixed-ef residency).
 #ifndef HNSWGPU_LEAN_MODEL_SMEM
 #define HNSWGPU_LEAN_MODEL_SMEM 1
 #endif

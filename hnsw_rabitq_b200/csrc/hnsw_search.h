@@ -164,7 +164,7 @@ size_t lean_smem_layout(SearchParams& p);
 // row a multiple of 32 and either <= 128 or a multiple of 128.
 bool lean_eligible(const SearchParams& p);
 cudaError_t launch_hnsw_lean(const SearchParams& p, int space, int num_sms, cudaStream_t stream, int* blocks_out);
-constexpr int kLeanWarpsPerBlock = 2;
+constexpr int kLeanWarpsPerBlock = 1;
 // learned-stop lean kernels: four query warps share one copy of the packed
 // network in shared memory
 constexpr int kLeanWarpsPerBlockLearned = 4;

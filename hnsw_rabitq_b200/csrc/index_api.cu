@@ -513,7 +513,8 @@ hnswgpu::SearchParams hnsw_params(const hnswgpu_index* h, const float* dq, uint6
     p.lean_w = p.maxM0 <= 32 ? 2u : 1u;
     // (the lean beam's learned-stop kernels, four warps per CTA beside one
     // copy of the network, are budgeted in apply_term)
-    const size_t wpb = p.lean ? hnswgpu::kLeanWarpsPerBlock : hnswgpu::kWarpsPerBlock;
+    // (the lean beam's limit on ef stays that of two query warps per CTA)
+    const size_t wpb = p.lean ? 2 : hnswgpu::kWarpsPerBlock;
     size_t ws = hnswgpu::warp_smem_layout(p);
     int max_optin = 0;
     cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attr");
