@@ -21,7 +21,7 @@
 // Measured, 5000 queries x 200k rows x 768 dims, bf16, k = 100 (device times
 // before -> after the sample was split over the SMs, the filter made
 // straight-line code and the list selected instead of sorted): threshold 183
-// -> 65 us, scores 1.95 -> 1.79 ms, selection and re-rank 2.42 -> 1.41 ms.
+// -> 65 us, scores 1.95 -> 1.20 ms, selection and re-rank 2.42 -> 1.41 ms.
 // A query whose list overflowed, or which found fewer than R candidates
 // below a sampled threshold, is answered by the exact kernel instead.
 //
@@ -29,7 +29,7 @@
 // K-major tiles, 4-stage ring), one thread of warp 1 issues the MMAs
 // (M=128, N=256, cta_group::1) and owns the TMEM allocation (two 256-column
 // accumulators, so the epilogue of one tile overlaps the MMAs of the next),
-// warps 2-5 drain TMEM (each warp its 32-lane quarter).  Every wait is
+// warps 2-9 drain TMEM (two warps per 32-lane quarter).  Every wait is
 // bounded; on a timeout the kernel raises a status bit and stops.
 #include <cuda.h>
 #include <cudaTypedefs.h>

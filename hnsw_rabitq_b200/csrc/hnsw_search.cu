@@ -6,8 +6,8 @@
 //
 // Per warp (= per query in flight) the shared memory holds
 //   * the query row,
-//   * a staging area that TMA bulk copies fill with the neighbour vectors of
-//     the node being expanded (one 16-byte aligned row per neighbour),
+//   * a staging area that TMA gathers of four rows (bulk copies for long rows)
+//     fill with the neighbour vectors of the node being expanded,
 //   * the candidate pool: up to ef (distance, id) keys sorted ascending, each
 //     with an "expanded" flag -- it plays the role of both of the reference's
 //     heaps (top_candidates and candidate_set, hnswalg.h:321-322),
@@ -28,9 +28,10 @@
 // either still in the pool / second list (found by exact key lookup and
 // skipped) or has d >= lowerBound and is rejected again, so cache misses cost
 // only a repeated distance, never a different result.  Ties in distance are
-// broken by internal id; on the same index the kernel therefore returns the
+// broken by internal id; on the same index the id order therefore returns the
 // reference's labels except where distances tie exactly (the oracle's
-// "canonical" mode computes exactly this kernel's result).
+// "canonical" mode computes exactly its result).  The tie-exact order (EXACT)
+// returns the reference's labels throughout.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>

@@ -545,8 +545,8 @@ class Index(_GpuIndex):
         upper distances, level-0 expansions, level-0 distances] and counts;
         no exception for short results.  tie_order "replay" gives the
         "reference" results by replaying the reference's heaps for every query
-        in one pass (the default reference order replays only the queries whose
-        id-order run met a steering tie)."""
+        (the default reference order replays only the queries whose id-order
+        run met a tie that can change the result)."""
         order = tie_order or self.tie_order
         if order not in ("reference", "id", "replay"):
             raise ValueError("tie_order must be 'reference', 'id' or 'replay'")
