@@ -46,6 +46,7 @@
 #include "launch_cache.h"
 #include "ref_heap.h"
 #include "term_mlp.cuh"
+#include "tie_rule.h"
 
 namespace hnswgpu {
 
@@ -727,28 +728,11 @@ __device__ __forceinline__ void term_final_row(const SearchParams& p, const Warp
     if (lane == 0) p.ckpt_count[qi] = r + 1;
 }
 
-// The tie-exact order (EXACT) without heaps.  Acceptance is by counting and does
-// not depend on heap layout, so a run in the (distance, id) order and the
-// reference's run differ only where distances tie, and most ties cannot change
-// the outcome:
-//   (a) The candidate popped next shares its distance d with another one.  Both
-//       runs then expand the tied candidates and everything they find at d or
-//       closer, in different orders, before they go beyond d.  If lowerBound
-//       is still above d when that is done, every one of these nodes was
-//       accepted and expanded in either order: lowerBound only falls as nodes
-//       are seen, so it was above d all along.  The same nodes have been seen,
-//       the pools hold the same distances, and what one run accepted and the
-//       other rejected lies beyond lowerBound, where a candidate can only end
-//       the search.  (A neighbour rejected meanwhile at exactly lowerBound
-//       could be such a difference: it counts as a tie that matters.)
-//   (b) The entry dropped from the full pool ties with its new worst entry.
-//       The reference may keep the other one, and both stay in its
-//       candidate_set; that matters only if candidates at that distance come up
-//       for expansion (or the search ends) while lowerBound is still there.
-//   (c) The k-th and the next result tie: the heap's layout decides.
-// A query that meets a tie that can matter is run again with the reference's
-// heaps, operation by operation (LIVE), by the same warp.  On 1M x 128 integer
-// vectors at ef 50, 11 % of the queries meet a tie of the three kinds and far
+// The tie-exact order (EXACT) starts without heaps: a run in the (distance, id)
+// order has the reference's result unless it meets a tie that can matter
+// (tie_rule.h).  A query that does is run again with the reference's heaps,
+// operation by operation (LIVE), by the same warp.  On 1M x 128 integer vectors
+// at ef 50, 11 % of the queries meet a tie of the rule's three kinds and far
 // fewer one that can matter.
 struct HeapState {
     bool live = false;  // the run keeps the reference's heaps
@@ -826,7 +810,7 @@ __device__ __forceinline__ int beam_loop(const SearchParams& p, WarpSmem& s, uin
     const int pcap = (int)p.pool_cap;
     int xsize = 0, hint_x = 0;  // FILTER: the list of disallowed candidates
     const int xcap = (int)p.extra_cap;
-    uint32_t tie_a = 0, tie_b = 0;  // EXACT: distances of the ties (a), (b) not settled yet (keys; 0: none)
+    TieRule tie;  // EXACT without heaps
     while (true) {
         float d;
         ct.l0_dists += b.f.nnew;
@@ -838,11 +822,11 @@ __device__ __forceinline__ int beam_loop(const SearchParams& p, WarpSmem& s, uin
         const bool full = psize == ef;
         const uint32_t lbk = full ? khi(s.pool[psize - 1]) : 0xffffffffu;
         bool live = f.fresh && !(full && dk >= lbk);
-        bool matters = EXACT && !LIVE && tie_a && __any_sync(FULL, f.fresh && full && dk == lbk);
+        const bool tie_open = EXACT && !LIVE && tie.open();
         uint64_t key = ((uint64_t)dk << 32) | f.id;
         int posP = 0, cntP = 0, posX = 0;
+        bool dup = false;  // already in the pool (or the list)
         if (live) {
-            bool dup = false;
             cntP = upper_bound_hi(s.pool, psize, dk);
             posP = insert_pos(s.pool, cntP, dk, f.id, dup);
             if (FILTER && !dup) posX = insert_pos(s.extra, upper_bound_hi(s.extra, xsize, dk), dk, f.id, dup);
@@ -919,7 +903,7 @@ __device__ __forceinline__ int beam_loop(const SearchParams& p, WarpSmem& s, uin
                         if (EXACT) {  // (a): candidate_set's top must be unique by distance
                             int same = __popc(__ballot_sync(FULL, accept && dk == next_dk));
                             if (ip >= 0) same += unexpanded_with_dist(s.pool, psize, ip, next_dk, lane);
-                            if (same > 1) tie_a = max(tie_a, next_dk);
+                            tie.picked(next_dk, same);
                         }
                         if (kmin < kp) {
                             next = (uint32_t)kmin;
@@ -958,23 +942,19 @@ __device__ __forceinline__ int beam_loop(const SearchParams& p, WarpSmem& s, uin
             const int m = merge_keys(s.pool, psize, pcap, put, key, posP, s.accbuf, na, lane);
             b.hint_p = min(b.hint_p, m);
             if (EXACT && !LIVE && psize > ef) {
-                if (khi(s.pool[ef]) == khi(s.pool[ef - 1])) tie_b = khi(s.pool[ef]);
+                tie.dropped(khi(s.pool[ef]), khi(s.pool[ef - 1]));
                 psize = ef;
             }
             if (LIVE && nev) psize = remove_keys(s.pool, psize, s.evbuf, nev, lane);
         }
-        if (EXACT && !LIVE && (tie_a | tie_b) && !inner) {
-            // settle the open ties against lowerBound after this expansion
-            const uint32_t lb = psize == ef ? khi(s.pool[ef - 1]) : 0xffffffffu;
-            const uint32_t nd = have_next ? next_dk : 0xffffffffu;
-            if (tie_a && nd > tie_a) {
-                matters |= lb <= tie_a;
-                tie_a = 0;
-            }
-            if (lb < tie_b) tie_b = 0;
-            matters |= tie_b && nd >= tie_b;
+        if (EXACT && !LIVE && (tie_open || tie.a || tie.b)) {
+            // neighbours of this unit left out at the bound it leaves behind, and
+            // the open ties against that bound after the whole expansion
+            const uint32_t lb = psize == ef ? khi(s.pool[ef - 1]) : TieRule::kNoBound;
+            if (tie_open && psize == ef && __any_sync(FULL, f.fresh && !accept && !dup && dk == lb)) tie.rejected();
+            if (!inner) tie.settle(lb, have_next ? next_dk : TieRule::kNoBound);
         }
-        if (EXACT && !LIVE && matters) {
+        if (EXACT && !LIVE && tie.matters) {
             if (have_next && fn.n0 > 0) copies_done(s, phase);
             return kBeamTie;
         }
