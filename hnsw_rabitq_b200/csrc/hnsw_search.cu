@@ -1713,6 +1713,21 @@ cudaError_t launch_term(const SearchParams& p, int num_sms, cudaStream_t stream,
 }
 }  // namespace
 
+cudaError_t exact_resident_ctas(int* out) {
+    const void* fns[] = {(const void*)hnsw_search_kernel<0, true, true, 0, 0, false>,
+                         (const void*)hnsw_search_kernel<0, false, true, 0, 0, false>,
+                         (const void*)hnsw_search_kernel<1, true, true, 0, 0, false>,
+                         (const void*)hnsw_search_kernel<1, false, true, 0, 0, false>};
+    *out = 1;
+    for (const void* fn : fns) {
+        int ctas = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, fn, kWarpsPerBlock * 32, 0);
+        if (e != cudaSuccess) return e;
+        *out = std::max(*out, ctas);
+    }
+    return cudaSuccess;
+}
+
 #ifdef HNSWGPU_BOUNDS_CHECK
 cudaError_t read_debug_record(unsigned long long* out) {
     cudaError_t e = cudaMemcpyFromSymbol(out, g_dbg, sizeof(unsigned long long) * 8);

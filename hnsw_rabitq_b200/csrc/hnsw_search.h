@@ -153,6 +153,9 @@ cudaError_t noalloc_scratch_address(int device, uint32_t** out);
 // *status (device memory).
 cudaError_t launch_wait_timeout_selftest(uint32_t limit, uint32_t* status, cudaStream_t stream);
 
+// CTAs of the tie-exact kernels that can reside on an SM, whatever shared
+// memory a launch takes.
+cudaError_t exact_resident_ctas(int* out);
 // Whether an unfiltered search runs in the pipelined beam.
 bool hnsw_pipelined(const SearchParams& p);
 // Fills the off_* fields and warp_smem from the sizes; returns warp_smem.

@@ -575,17 +575,45 @@ void apply_term(const hnswgpu_index* h, hnswgpu::SearchParams& p, const TermCfg*
     }
 }
 
-// Global tails of the tie-exact candidate heaps, one per resident warp (at
-// most 32 CTAs per SM), owned by the index.
-static void attach_spill(hnswgpu_index* h, hnswgpu::SearchParams& p, cudaStream_t st) {
-    const uint64_t warps = (uint64_t)h->num_sms * 32u * hnswgpu::kWarpsPerBlock;
-    const uint64_t need = warps * p.cand_spill_cap;
-    if (h->cand_spill.n < need) {
-        cuda_check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
-        h->cand_spill.alloc(need);
+// Global tails of the tie-exact candidate heaps, one per resident warp, owned
+// by the index.  Sized by ef alone (whole heaps but for their kHeapHead first
+// entries, as many warps as the registers of those kernels let reside), never by
+// the batch: a stream capture keeps the pointer, so a block that one has seen is
+// kept until the index is freed.  The launches that use the block are ordered on
+// the GPU by an event, whichever streams they are on (spill_used); a capturing
+// stream cannot wait for it and is left out.  Returns whether `st` is capturing.
+constexpr uint32_t kHeapHead = 32;
+static bool attach_spill(hnswgpu_index* h, hnswgpu::SearchParams& p, cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cuda_check(cudaStreamIsCapturing(st, &cs), "cudaStreamIsCapturing");
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    if (!h->exact_ctas) cuda_check(hnswgpu::exact_resident_ctas(&h->exact_ctas), "occupancy");
+    const uint64_t warps = (uint64_t)h->num_sms * (uint64_t)h->exact_ctas * hnswgpu::kWarpsPerBlock;
+    const uint64_t need = warps * ((uint64_t)p.cand_cap + p.cand_spill_cap);
+    if (h->cand_spill->n < need) {
+        if (capturing)
+            throw ApiError(HNSWGPU_ERR_STATE, "make one such call (same ef) on this index before capturing it");
+        if (h->spill_captured) {
+            h->spill_kept.push_back(std::move(h->cand_spill));
+            h->cand_spill.reset(new DevBuf<uint64_t>());
+            h->spill_captured = false;
+        } else if (h->spill_pending) {
+            cuda_check(cudaEventSynchronize(h->spill_ev), "cudaEventSynchronize");
+        }
+        h->cand_spill->alloc(need);
     }
-    p.cand_spill = h->cand_spill.p;
+    if (capturing) h->spill_captured = true;
+    else if (h->spill_pending) cuda_check(cudaStreamWaitEvent(st, h->spill_ev, 0), "cudaStreamWaitEvent");
+    p.cand_spill = h->cand_spill->p;
     p.cand_spill_warps = (uint32_t)warps;
+    return capturing;
+}
+
+// A launch on `st` that the caller does not wait for now uses the spill block.
+static void spill_used(hnswgpu_index* h, cudaStream_t st) {
+    if (!h->spill_ev) cuda_check(cudaEventCreateWithFlags(&h->spill_ev, cudaEventDisableTiming), "cudaEventCreate");
+    cuda_check(cudaEventRecord(h->spill_ev, st), "cudaEventRecord");
+    h->spill_pending = true;
 }
 
 static void take_counter_slot(hnswgpu_index* h, hnswgpu::SearchParams& p) {
@@ -625,6 +653,7 @@ void run_hnsw(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint64
     apply_term(h, p, term);
     p.status = h->status.p;
     const int space = kspace(h);
+    const bool capturing = exact && attach_spill(h, p, st);
     if (exact && !replay_all && p.bare && hnswgpu::hnsw_pipelined(p)) {
         p.lazy_heaps = 1u;
         if (nq > 8ull * (uint64_t)h->num_sms) {
@@ -632,13 +661,12 @@ void run_hnsw(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint64
             // heap goes to the spill area, for the sake of residency (a small
             // batch waits for the slowest query, heaps and all)
             const uint32_t cap = p.cand_cap + p.cand_spill_cap;
-            p.cand_cap = std::min(p.cand_cap, 32u);
+            p.cand_cap = std::min(p.cand_cap, kHeapHead);
             p.cand_spill_cap = cap - p.cand_cap;
             hnswgpu::warp_smem_layout(p);
         }
     }
     if (wide) widen_staging(h, p, nq);
-    if (exact) attach_spill(h, p, st);
 #ifdef HNSWGPU_PHASE_TIMING
     static unsigned long long* phase_buf = nullptr;
     if (!phase_buf) {
@@ -650,6 +678,7 @@ void run_hnsw(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, uint64
 #endif
     take_counter_slot(h, p);
     cuda_check(hnswgpu::launch_hnsw_search(p, space, h->num_sms, st, nullptr), "hnsw_search launch");
+    if (exact && !wide && !capturing) spill_used(h, st);
 }
 
 // Epsilon search of a batch on device buffers: searchStopConditionClosest
@@ -676,10 +705,11 @@ void run_epsilon(hnswgpu_index* h, const float* dq, uint64_t nq, float eps, uint
     p.eps = eps;
     p.eps_min = (uint32_t)min_c;
     p.status = h->status.p;
-    attach_spill(h, p, st);
+    const bool capturing = attach_spill(h, p, st);
     take_counter_slot(h, p);
     cuda_check(hnswgpu::launch_hnsw_search(p, kspace(h), h->num_sms, st, nullptr),
                "hnsw_search launch");
+    if (!capturing) spill_used(h, st);
 }
 
 // Stream-ordered workspace of one call from the index's own pool: freed on

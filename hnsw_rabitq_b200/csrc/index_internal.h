@@ -91,7 +91,13 @@ struct hnswgpu_index {
     DevBuf<float> bf_norms;    // brute force: per-row helper values
     DevBuf<unsigned char> tcopy[3];  // low-precision traversal copies (index 1 bf16, 2 fp8)
     DevBuf<unsigned char> term_model;  // learned termination: packed network
-    DevBuf<uint64_t> cand_spill;       // tie-exact mode: candidate-heap tails
+    // tie-exact mode: candidate-heap tails; blocks that a stream capture refers
+    // to, and the last launch that is not waited for by its caller
+    std::unique_ptr<DevBuf<uint64_t>> cand_spill{new DevBuf<uint64_t>()};
+    std::vector<std::unique_ptr<DevBuf<uint64_t>>> spill_kept;
+    cudaEvent_t spill_ev = nullptr;
+    int exact_ctas = 0;  // resident CTAs per SM of the tie-exact kernels, at most
+    bool spill_captured = false, spill_pending = false;
     DevBuf<float2> tc_rowinfo[3];      // tensor-core brute force: (|x|^2, scale) per row and precision
     // tensor-core brute force: per-call workspace
     DevBuf<float> tc_qf, tc_qscale, tc_tau, tc_part;
@@ -111,6 +117,7 @@ struct hnswgpu_index {
     // search can hold it while it reads that state
     mutable std::mutex mu;
     ~hnswgpu_index() {
+        if (spill_ev) cudaEventDestroy(spill_ev);
         if (pinned) cudaFreeHost(pinned);
         if (pool) cudaMemPoolDestroy(pool);
     }

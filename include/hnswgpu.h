@@ -61,11 +61,13 @@ extern "C" {
                                      copies, launches and synchronises.
                                      Tie-exact searches (HNSWGPU_EXACT_TIES,
                                      hnswgpu_search_epsilon) of one index share
-                                     its scratch (candidate-heap tails, the tie
-                                     list): asynchronous ones must not overlap
-                                     on the GPU, so issue them on one stream or
-                                     order their streams (the serving loop runs
-                                     one at a time).                            */
+                                     its scratch (candidate-heap tails, sized by
+                                     ef): calls on several streams run one
+                                     after the other on the GPU.  A captured
+                                     one needs an earlier call at its ef or a
+                                     larger one, and its replays must not
+                                     overlap another tie-exact search of the
+                                     index.                                     */
 #define HNSWGPU_TRACE 0x2u        /* write per-query work counters to `trace`   */
 #define HNSWGPU_EXACT_TIES 0x4u   /* HNSW: replay the reference's heap order so
                                      that exact distance ties resolve as in
