@@ -44,6 +44,7 @@
 #include "bf_tc.h"
 #include "device_common.cuh"
 #include "hnsw_search.h"
+#include "launch_cache.h"
 
 namespace hnswgpu {
 namespace {
@@ -1208,7 +1209,9 @@ cudaError_t launch_tc_select(const TcSelectArgs& a, int space, cudaStream_t st) 
     if (!a.nq) return cudaSuccess;
     const size_t smem = tc_select_smem(a.sort_cap, a.dim, a.R);
     auto fn = space == 0 ? tc_select_rerank_kernel<0> : tc_select_rerank_kernel<1>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static LaunchCache cache[2];
+    int occ = 0;
+    cudaError_t e = cache[space != 0].blocks_per_sm((const void*)fn, kSelThreads, smem, &occ);
     if (e != cudaSuccess) return e;
     fn<<<a.nq, kSelThreads, smem, st>>>(a);
     return cudaGetLastError();
@@ -1222,7 +1225,9 @@ cudaError_t launch_tc_certify(const TcCertArgs& a, int space, cudaStream_t st) {
     if (!a.nq) return cudaSuccess;
     const size_t smem = tc_certify_smem(a.cap, a.dim);
     auto fn = space == 0 ? tc_certify_kernel<0> : tc_certify_kernel<1>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static LaunchCache cache[2];
+    int occ = 0;
+    cudaError_t e = cache[space != 0].blocks_per_sm((const void*)fn, kSelThreads, smem, &occ);
     if (e != cudaSuccess) return e;
     fn<<<a.nq, kSelThreads, smem, st>>>(a);
     return cudaGetLastError();
