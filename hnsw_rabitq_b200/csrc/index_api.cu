@@ -754,10 +754,6 @@ static void run_bf_simt(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t
     b.out_labels = dl;
     b.out_dists = dd;
     b.out_counts = dc;
-    int max_optin = 0;
-    cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attr");
-    if (!hnswgpu::bf_supported(b.k, b.row_floats, (size_t)max_optin))
-        cuda_check(cudaErrorInvalidConfiguration, "bf_search launch");
     uint32_t batch = hnswgpu::bf_batch(b);
     PoolBuf ws(st);
     cudaError_t e = ws.alloc(h, hnswgpu::bf_workspace(b, batch));
@@ -948,6 +944,11 @@ static bool run_bf_certified(hnswgpu_index* h, const float* dq, uint64_t nq, uin
 // certified, so calls that only enqueue work keep the float32 kernels).
 static void run_bf_exact(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, const uint8_t* dallow,
                          uint64_t* dl, float* dd, int32_t* dc, cudaStream_t st, bool may_sync) {
+    // one limit for both routes: what one of them cannot answer the other must
+    int max_optin = 0;
+    cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attr");
+    if (!hnswgpu::bf_supported((uint32_t)k, h->row_floats, (size_t)max_optin))
+        cuda_check(cudaErrorInvalidConfiguration, "bf_search launch");
     if (may_sync && bf_tensor_exact(h->count, nq, k, h->dim) && run_bf_certified(h, dq, nq, k, dallow, dl, dd, dc, st))
         return;
     run_bf_simt(h, dq, nq, k, dallow, dl, dd, dc, st);
