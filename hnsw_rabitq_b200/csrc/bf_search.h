@@ -27,6 +27,17 @@ bool bf_supported(uint32_t k, uint32_t row_floats, size_t max_smem);
 // Queries of p that run at once, and the bytes of workspace for `batch` at once.
 uint32_t bf_batch(const BfParams& p);
 size_t bf_workspace(const BfParams& p, uint32_t batch);
+// Allocates for `batch` queries at once, fewer where memory is short: down to
+// one, whose keys are the least the scan can do with.
+template <class Alloc>
+cudaError_t bf_fit_batch(uint32_t& batch, Alloc alloc) {
+    cudaError_t e = alloc(batch);
+    while (e == cudaErrorMemoryAllocation && batch > 1) {
+        batch = batch / 4 > 1 ? batch / 4 : 1;
+        e = alloc(batch);
+    }
+    return e;
+}
 cudaError_t launch_bf_search(BfParams p, int space, void* workspace, uint32_t batch, cudaStream_t stream);
 
 }  // namespace hnswgpu

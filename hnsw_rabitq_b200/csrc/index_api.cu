@@ -756,12 +756,11 @@ static void run_bf_simt(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t
     b.out_counts = dc;
     uint32_t batch = hnswgpu::bf_batch(b);
     PoolBuf ws(st);
-    cudaError_t e = ws.alloc(h, hnswgpu::bf_workspace(b, batch));
-    while (e == cudaErrorMemoryAllocation && batch > 8) {  // little memory left: fewer queries at once
-        (void)cudaGetLastError();
-        batch = std::max(8u, batch / 4);
-        e = ws.alloc(h, hnswgpu::bf_workspace(b, batch));
-    }
+    const cudaError_t e = hnswgpu::bf_fit_batch(batch, [&](uint32_t m) {
+        const cudaError_t a = ws.alloc(h, hnswgpu::bf_workspace(b, m));
+        if (a == cudaErrorMemoryAllocation) (void)cudaGetLastError();
+        return a;
+    });
     cuda_check(e, "bf_search workspace");
     cuda_check(hnswgpu::launch_bf_search(b, kspace(h), ws.p, batch, st), "bf_search launch");
 }
