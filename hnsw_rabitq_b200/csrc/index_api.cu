@@ -714,7 +714,10 @@ void run_epsilon(hnswgpu_index* h, const float* dq, uint64_t nq, float eps, uint
 
 // Stream-ordered workspace of one call from the index's own pool: freed on
 // the stream that used it, so calls on several streams never share a block.
-// The pool keeps its peak for the next call until the index is freed.
+// The pool keeps at most kPoolKeep between calls (a certified scan of 2048
+// queries with k > 100 takes 210 MB), all of it until the index is freed; what a
+// larger call took goes back when its stream is waited for.
+constexpr uint64_t kPoolKeep = 256ull << 20;
 struct PoolBuf {
     void* p = nullptr;
     cudaStream_t st;
@@ -726,14 +729,16 @@ struct PoolBuf {
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = h->device;
             cuda_check(cudaMemPoolCreate(&h->pool, &props), "cudaMemPoolCreate");
-            uint64_t keep = ~0ull;
+            uint64_t keep = kPoolKeep;
             cuda_check(cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
         }
         return cudaMallocFromPoolAsync(&p, bytes, h->pool, st);
     }
-    ~PoolBuf() {
+    void free() {
         if (p) cudaFreeAsync(p, st);
+        p = nullptr;
     }
+    ~PoolBuf() { free(); }
 };
 
 // Exact brute force of a batch on device buffers by the float32 kernels
@@ -934,6 +939,7 @@ static bool run_bf_certified(hnswgpu_index* h, const float* dq, uint64_t nq, uin
     std::vector<uint32_t> redo;
     for (uint64_t i = 0; i < nq; i++)
         if (flags[i]) redo.push_back((uint32_t)i);
+    ws.free();  // (the float32 kernels need their own)
     if (!redo.empty()) redo_exact(h, dq, redo, k, dallow, dl, dd, dc, st, false);
     return true;
 }

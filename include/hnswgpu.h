@@ -114,7 +114,14 @@ typedef struct hnswgpu_info {
     uint32_t enterpoint;
     int32_t space;
     int32_t is_bruteforce;
-    uint64_t device_bytes;     /* bytes of index data resident on the GPU       */
+    uint64_t device_bytes;     /* bytes of index data resident on the GPU: rows,
+                                  links, labels, and the bf16 / fp8 copies of
+                                  the rows once a call has built them (exact
+                                  scans of large host batches build the bf16
+                                  copy too, if there is memory for it).  Not
+                                  counted: scratch kept between calls, such as
+                                  up to 256 MB of scan workspace and the
+                                  heap tails of tie-exact searches            */
 } hnswgpu_info;
 
 typedef struct hnswgpu_search_opts {
