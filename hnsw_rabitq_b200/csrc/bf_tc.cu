@@ -42,6 +42,7 @@
 #include <cstdint>
 
 #include "bf_tc.h"
+#include "cert_bound.h"
 #include "device_common.cuh"
 #include "hnsw_search.h"
 #include "launch_cache.h"
@@ -642,21 +643,8 @@ __global__ void tc_query_prep_kernel(const float* __restrict__ q, uint32_t nq, u
             e += __shfl_xor_sync(0xffffffffu, e, of);
         }
         if (lane == 0) {
-            // How far the tensor-core distance of any row may lie from the
-            // reference's float32 distance.  |q.x - q'.x'| <= |q - q'||x| +
-            // |q'||x - x'| for the rounded q', x' (Cauchy-Schwarz); the
-            // tensor cores' float32 accumulation: 2^-21 |q'||x'| per 16
-            // products and 32 of them over (several times an accumulation
-            // that truncates at 24 bits); the reference's own summation and
-            // the norms, at most dim / 4 + 64 roundings of 2^-24: twice that.
-            // Subnormal inputs the tensor cores may drop: the 2^-126 term.
             const double nq = sqrt((double)s) * 1.001, dq = sqrt((double)e) * 1.001;
-            const double M = __uint_as_float(stats[0]), D = __uint_as_float(stats[1]);
-            const double eps = 1.0 / (1 << 23);
-            const double E = dq * M + (nq + dq) * D + (dim / 16 + 32) * 4.0 * eps * (nq + dq) * (M + D) +
-                             (nq + M + 1.0) * dim * 1.2e-38;
-            const double g = (dim / 4 + 64) * eps;
-            const double B = space == 0 ? 2.0 * E + g * (nq + M) * (nq + M) : E + g * nq * M + 2.0 * eps * (1.0 + nq * M);
+            const double B = cert_bound(space, dim, nq, dq, __uint_as_float(stats[0]), __uint_as_float(stats[1]));
             qinfo[row] = make_float2(space == 0 ? s : 1.f, (float)(B * 1.001));
         }
         return;
