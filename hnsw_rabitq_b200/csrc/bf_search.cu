@@ -138,9 +138,13 @@ struct DistSmem {
     float q[kStages][QT * kKC];
 };
 
-// Distance keys of 128 rows x QT queries.  Bound by the shared-memory reads
-// (per 16 elements: 16 wavefronts for the row, 4 QT for the queries against
-// 16 QT FMA instructions over four schedulers) for a batch, by HBM for QT = 1.
+// Distance keys of 128 rows x QT queries.  QT = 1 is bound by the loads in
+// flight (400k x 100: 34 us, 4.85 TB/s, 74 % of a copy's rate; 15 warps an SM by
+// shared memory, 3.5 cycles an issue on global loads).  QT = 8 fills no unit: 100
+// queries x 100k x 128 take 226 us with 59 % of the issue slots and 47 % of the
+// shared-memory pipe (per 16 elements 16 wavefronts for the row and 4 QT for the
+// queries, beside 16 QT FMA and, for L2, 16 QT subtractions); 205 registers and 58
+// KB leave 8 warps an SM to hide their latencies.
 template <int SPACE, int FORM, int QT>
 __global__ void __launch_bounds__(kRows) bf_dist_kernel(BfParams p) {
     extern __shared__ __align__(16) unsigned char raw[];

@@ -257,41 +257,6 @@ __device__ __forceinline__ float dist_ip(const float* q, const float* x, int dim
     return __fsub_rn(1.0f, ip_scalar(q, x, dim));
 }
 
-template <int SPACE>
-__device__ __forceinline__ float group4_reduce(float c0, float c1, float c2, float c3);
-
-// The dim % 16 == 0 distance split over a group of 4 lanes (a = lane & 3):
-// lane a keeps the reference's accumulators 4a .. 4a+3 (one float4 of each
-// 16-float chunk), so one LDS.128 per chunk per lane feeds 8 vectors per warp
-// instruction.  The cross-lane reduction reproduces the reference order
-// exactly: L2 sums the 16 accumulators left to right (space_l2.h:49-51), IP
-// applies GCC's _mm512_reduce_add_ps tree then 1 - x.  All 32 lanes must call
-// it (it shuffles); the result is valid in lanes with a == 0.
-template <int SPACE>
-__device__ __forceinline__ float group4_dist16(const float* __restrict__ q, const float* __restrict__ x, int n16,
-                                               int a) {
-    const float4* q4 = reinterpret_cast<const float4*>(q);
-    const float4* x4 = reinterpret_cast<const float4*>(x);
-    float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
-    for (int c = 0; c < n16; c++) {
-        float4 qv = q4[4 * c + a], xv = x4[4 * c + a];
-        if (SPACE == 0) {
-            float t0 = __fsub_rn(qv.x, xv.x), t1 = __fsub_rn(qv.y, xv.y), t2 = __fsub_rn(qv.z, xv.z),
-                  t3 = __fsub_rn(qv.w, xv.w);
-            c0 = __fmaf_rn(t0, t0, c0);
-            c1 = __fmaf_rn(t1, t1, c1);
-            c2 = __fmaf_rn(t2, t2, c2);
-            c3 = __fmaf_rn(t3, t3, c3);
-        } else {
-            c0 = __fmaf_rn(qv.x, xv.x, c0);
-            c1 = __fmaf_rn(qv.y, xv.y, c1);
-            c2 = __fmaf_rn(qv.z, xv.z, c2);
-            c3 = __fmaf_rn(qv.w, xv.w, c3);
-        }
-    }
-    return group4_reduce<SPACE>(c0, c1, c2, c3);
-}
-
 // GCC's _mm512_reduce_add_ps tree over the 16 accumulators of a 4-lane group.
 __device__ __forceinline__ float group4_ip_sum(float c0, float c1, float c2, float c3) {
     // T3[i] = a[i+8] + a[i]: lanes 0,1 pair with lanes 2,3
@@ -307,8 +272,13 @@ __device__ __forceinline__ float group4_ip_sum(float c0, float c1, float c2, flo
     return __fadd_rn(__fadd_rn(v0, v2), __fadd_rn(v1, v3));
 }
 
-// Cross-lane reduction of group4_dist16: lane a of a 4-lane group holds the
-// reference's accumulators 4a .. 4a+3.
+// Cross-lane reduction of a dim % 16 == 0 distance split over a group of 4
+// lanes: lane a holds the reference's accumulators 4a .. 4a+3 (one float4 of
+// each 16-float chunk, so one LDS.128 per chunk per lane feeds 8 vectors per warp
+// instruction).  In the reference's order: L2 sums the 16 accumulators left to
+// right (space_l2.h:49-51), IP applies GCC's _mm512_reduce_add_ps tree then
+// 1 - x.  All 32 lanes must call it (it shuffles); the result is valid in lanes
+// with a == 0.
 template <int SPACE>
 __device__ __forceinline__ float group4_reduce(float c0, float c1, float c2, float c3) {
     if (SPACE == 0) {

@@ -49,8 +49,9 @@
 // launch bound, resident 1-warp CTAs per SM (96 registers, 20 query warps
 // reside).  One warp per CTA instead of two: a CTA gives its shared memory back
 // when its own query is done (500k x 128, ef 52, a call: 100 queries 233 -> 224
-// us, 10k 1.30 -> 1.28 ms).  Bounds of 16 and 20 were 7 % and 3 % slower than
-// 18: the compiler schedules the loop differently for each.
+// us; 10k queries 1279-1346 -> 1282-1331 us, no difference to see).  Bounds of
+// 16 and 20 were 7 % and 3 % slower than 18: the compiler schedules the loop
+// differently for each.
 #ifndef HNSWGPU_MINB_LEAN
 #define HNSWGPU_MINB_LEAN 18
 #endif

@@ -815,11 +815,13 @@ static bool bf_tensor_exact(uint64_t n, uint64_t nq, uint64_t k, uint64_t dim) {
 }
 
 // Exact brute force through the tensor cores: bf16 scores of all rows choose
-// the candidates, exact float32 distances of these decide, and a rigorous bound
-// on the scores' error certifies that no other row can belong to the answer
-// (tc_certify_kernel).  Queries it cannot certify go to the float32 kernels.
+// the candidates, exact float32 distances of these decide, and a bound on the
+// scores' error (cert_bound.h) certifies that no other row can belong to the
+// answer (tc_certify_kernel).  Queries it cannot certify go to the float32 kernels.
 // 500 queries x 200k rows x 768 dims, k = 100: 9.9 ms by the float32 kernels,
-// 0.62 ms here (scores 0.17, certification 0.15, the copies).  False when there is no memory for the bf16 copy.  Synchronises.
+// 0.61 ms here (scores 0.17, certification 0.11, the copies).  The bf16 copy of
+// the rows is built by the first such call and kept; false when there is no
+// memory for it.  Synchronises.
 static bool run_bf_certified(hnswgpu_index* h, const float* dq, uint64_t nq, uint64_t k, const uint8_t* dallow,
                              uint64_t* dl, float* dd, int32_t* dc, cudaStream_t st) {
     const uint64_t n = h->count;

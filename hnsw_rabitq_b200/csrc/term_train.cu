@@ -12,9 +12,11 @@
 // sample for the forward and the activation gradients (activations kept in
 // shared memory, rows padded to 65 floats so the per-sample rows fall in
 // distinct banks); then each CTA reduces a quarter of the weight gradients over
-// the samples into the tile's partial-gradient row.  term_adam_kernel sums the rows in a fixed order
-// (deterministic) and applies Adam.  The sizes are tiny (4.7k parameters),
-// so CUDA cores, not tensor cores, do this work.
+// the samples into the tile's partial-gradient row.  term_epoch_kernel runs a
+// whole epoch of such steps in one cooperative launch: after each batch's
+// gradients it sums the rows in a fixed order (deterministic) and applies Adam.
+// The sizes are tiny (4.7k parameters), so CUDA cores, not tensor cores, do this
+// work.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -355,7 +357,9 @@ __device__ __forceinline__ bool grid_meet(const TrainArgs& a, uint32_t gen) {
 }
 
 // One epoch in one cooperative launch: a step (gradient tiles, then Adam) is
-// about 20 us, and two launches a step cost as much again on a slow host.
+// 20-27 us, and two launches a step cost as much again on a slow host.  Bound by
+// one tile's latency: 32 of 148 SMs, 16 warps each, waits for shared memory (3.6
+// cycles an issue) and at barriers (2.3).
 __global__ void __launch_bounds__(kGradThreads) term_epoch_kernel(TrainArgs a) {
     extern __shared__ __align__(16) unsigned char raw[];
     TrainSmem& s = *reinterpret_cast<TrainSmem*>(raw);
