@@ -1626,6 +1626,22 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, PREC ? HNSWGPU_MINB_LOWP 
 
 bool hnsw_pipelined(const SearchParams& p) { return pipelined(p, false, p.fast16 != 0, (int)p.term_mode); }
 
+bool ef_supported(const SearchParams& p, size_t budget) {
+    auto up = [](size_t v, size_t to) { return (v + to - 1) / to * to; };
+    const size_t stride = ((size_t)p.row_floats + (p.fast16 ? 16 : 4)) * 4;
+    const size_t most = p.prec ? 8 : p.fast16 ? 16 : 32;
+    size_t stage = std::max<size_t>(1, std::min<size_t>(most, 9728 / stride)) * stride;
+    if (p.prec) stage = std::max(8 * stride, (size_t)p.tslots * p.tstage_bytes);
+    size_t bytes = up(up(144 + (size_t)p.row_floats * 4, 16) + up(stage, 16) + (4u << 8), 8) + (size_t)p.pool_cap * 8 +
+                   (size_t)p.extra_cap * 8;
+    if (p.exact) {
+        size_t head = p.cand_cap;
+        while (head > 4ull * p.ef) head -= p.ef;
+        bytes += ((size_t)p.ef + 1 + head + 64) * 8;
+    }
+    return up(bytes, 128) <= budget;
+}
+
 size_t warp_smem_layout(SearchParams& p) {
     if (p.lean) return lean_smem_layout(p);
     size_t off = 16 + 128;  // mbarrier (8 bytes) + pad, then the 32-entry id compaction buffer

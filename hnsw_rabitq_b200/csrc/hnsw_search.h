@@ -160,6 +160,12 @@ cudaError_t exact_resident_ctas(int* out);
 bool hnsw_pipelined(const SearchParams& p);
 // Fills the off_* fields and warp_smem from the sizes; returns warp_smem.
 size_t warp_smem_layout(SearchParams& p);
+// The interface's limit on ef (with the dimension, tie order, filter and
+// precision; not for the lean beam): a fixed function of these -- the bytes of a
+// query's state with rows staged at their width + 16 floats (+ 4 where dim % 16
+// != 0), a visited cache of 2^8 ids and, for the reference order, a heap head of
+// about 4 ef -- kept although the present layout differs.
+bool ef_supported(const SearchParams& p, size_t budget);
 // The lean fp8 beam's per-warp layout (called by warp_smem_layout when p.lean).
 size_t lean_smem_layout(SearchParams& p);
 // Whether the lean fp8 beam can run these parameters: fp8 copy, id tie order,

@@ -518,12 +518,21 @@ hnswgpu::SearchParams hnsw_params(const hnswgpu_index* h, const float* dq, uint6
     size_t ws = hnswgpu::warp_smem_layout(p);
     int max_optin = 0;
     cuda_check(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device), "attr");
+    if (p.lean ? ws * wpb > (size_t)max_optin : !hnswgpu::ef_supported(p, (size_t)max_optin / wpb))
+        throw ApiError(HNSWGPU_ERR_UNSUPPORTED, "ef too large for the per-query shared-memory budget");
+    // near that limit: a smaller visited cache, a smaller heap head, fewer
+    // staging slots
     while (!p.lean && ws * wpb > (size_t)max_optin && p.log2_vis > 7) {
         p.log2_vis--;
         ws = hnswgpu::warp_smem_layout(p);
     }
     while (exact && ws * wpb > (size_t)max_optin && p.cand_cap > 4u * p.ef) {
         p.cand_cap -= p.ef;
+        ws = hnswgpu::warp_smem_layout(p);
+    }
+    const uint32_t group = p.gather ? 4u : 1u;
+    while (!p.lean && !p.prec && ws * wpb > (size_t)max_optin && p.stage_slots > group) {
+        p.stage_slots -= group;
         ws = hnswgpu::warp_smem_layout(p);
     }
     if (ws * wpb > (size_t)max_optin)
